@@ -103,7 +103,7 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
-T1_FORMS = {1: "compact (one block per warp)", 2: "unrolled (one block per warp)", 3: "lanes (one block per lane)"}
+T1_FORMS = {1: "compact (one block per warp)", 2: "latency (one block per warp)", 3: "lanes (one block per lane)"}
 
 
 def measured_peaks():
@@ -788,7 +788,7 @@ def main():
     ap.add_argument("--decode-repeat", type=int, default=0,
                     help="profiling mode: decode the workload this many times, print stage times, no bench line")
     ap.add_argument("--frames", type=int, default=0, help="profiling mode: only the first N pictures")
-    ap.add_argument("--t1-form", type=int, default=0, help="profiling mode: Tier-1 form 0 auto, 1 compact, 2 unrolled, 3 lanes")
+    ap.add_argument("--t1-form", type=int, default=0, help="profiling mode: Tier-1 form 0 auto, 1 compact, 2 latency, 3 lanes")
     ap.add_argument("--dwt-coarse", type=int, default=0,
                     help="profiling mode: coarse DWT levels 0 auto, 1 fused into one kernel, 2 one launch per level")
     args = ap.parse_args()

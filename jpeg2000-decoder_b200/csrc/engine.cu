@@ -50,41 +50,36 @@ __device__ __forceinline__ int32_t place53(int32_t v, int numbps) {
   return v < 0 ? -(int32_t)((uint32_t)(v & 0x7FFFFFFF) >> sh) : (int32_t)((uint32_t)v >> sh);
 }
 
-template <int MAXW, int MAXH>
-struct T1Layout {
-  static constexpr int STRIPES = MAXH / 4;
-  static constexpr int GAP = MAXW + 3;
-  static constexpr int CWN = (STRIPES + 2) * GAP + 2;
-  static constexpr int RF_BYTES = ((STRIPES * GAP) + 3) & ~3;
-  // context words, refined bits, MQ context slots, then 32 bytes of per-chunk row masks
-  static constexpr int PER_WARP = ((CWN * 4 + RF_BYTES + N_CTX * 8 + 32) + 15) & ~15;
-};
-
 // Host-side queue classes: blocks the lane form decodes (up to 64x64, no bypass segments;
 // filled only when the batch is staged with t1_form 3) and the others; the warp forms take
 // both, as one queue (the two are contiguous), so without the lane form it is one queue
 // sorted longest first.
 enum { QL = 0, QW = 1, NQ = 2 };
-// The warp forms' tables (MQ states, zero-coding / sign contexts, bypass refinement
-// scatter) in constant memory: every lane of a warp reads the same entry, so the constant
-// cache broadcasts it, and the loads need no shared-memory copy per CTA.
-__constant__ T1Tables c_t1tables;
+// The warp forms' tables (MQ states, zero-coding / sign contexts), copied to shared memory by
+// every CTA
+__device__ T1Tables g_t1tables;
 
-template <int MAXW, int MAXH, bool UNROLLED>
+template <int MAXW, int MAXH, bool LATENCY>
 __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const uint32_t *__restrict__ order, int n,
                                         int *__restrict__ counter, const uint8_t *__restrict__ bytes,
                                         const uint32_t *__restrict__ seglens, void *__restrict__ coef,
                                         uint16_t *__restrict__ status) {
   extern __shared__ __align__(16) uint8_t smem[];
   typedef T1Layout<MAXW, MAXH> Lay;
-  const T1Tables &T = c_t1tables;
+  T1Tables &T = *reinterpret_cast<T1Tables *>(smem);
+  for (int i = threadIdx.x; i < (int)(sizeof(T1Tables) / 16); i += blockDim.x)
+    reinterpret_cast<uint4 *>(smem)[i] = reinterpret_cast<const uint4 *>(&g_t1tables)[i];
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t *mine = smem + warp * Lay::PER_WARP;
-  BlockSmem b;
-  b.cw = reinterpret_cast<uint32_t *>(mine);
-  b.rf = mine + Lay::CWN * 4;
-  b.cx = reinterpret_cast<uint2 *>(mine + Lay::CWN * 4 + Lay::RF_BYTES);
-  b.sp.lane = lane;
+  uint8_t *mine = smem + sizeof(T1Tables) + warp * Lay::PER_WARP;
+  Block b;
+  b.rf = reinterpret_cast<uint4 *>(mine + Lay::RF);
+  b.cx = mine + Lay::CX;
+  b.bits = reinterpret_cast<uint32_t *>(mine + Lay::BITS);
+  b.list = mine + Lay::LIST;
+  b.mq = reinterpret_cast<const uint8_t *>(T.mq);
+  b.sc = T.sc;
+  b.lane = lane;
   for (;;) {
     int idx = 0;
     if (lane == 0) idx = atomicAdd(counter, 1);
@@ -94,16 +89,19 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
     const j2k_cblk cb = cbs[ci];
     b.w = cb.w;
     b.gap = cb.w + 3;
+    b.stripes = (cb.h + 3) >> 2;
+    b.cw = reinterpret_cast<uint32_t *>(mine) + b.gap + 1;
+    b.zc = T.zc[cb.band == 3 ? 2 : (cb.band == 1 ? 1 : 0)];
     int32_t *blk = reinterpret_cast<int32_t *>(coef) + cb.out_off;
-    b.sp.base = blk;
-    b.sp.stride = cb.out_stride;
+    b.out = reinterpret_cast<uint32_t *>(blk);
+    b.stride = cb.out_stride;
     int bit_plane, num_passes;
     block_planes(cb, bit_plane, num_passes);
     int st;
     if (cb.w == 0 || cb.h == 0 || cb.w > MAXW || cb.h > MAXH) {
       st = 9;
     } else {
-      st = decode_block<UNROLLED>(cb, bytes, seglens, b, T, lane, bit_plane, num_passes);
+      st = decode_block<LATENCY>(cb, bytes, seglens, b, bit_plane, num_passes);
     }
     // rewrite the block in place: raw sign-magnitude -> dequantised float (9/7) or shifted
     // integer (5/3); the lanes' sample writes are made visible first.  A sample whose
@@ -115,8 +113,8 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
       const bool irrev = (cb.flags & J2K_CB_IRREV) != 0;
       for (int y = 0; y < h; ++y) {
         int32_t *r = blk + (size_t)y * cb.out_stride;
-        const uint32_t sig = ROW_SIG(y & 3);
-        const uint32_t *wrow = cword(b, y >> 2, 0);
+        const uint32_t sig = 1u << (SIG_POS + 3 * (y & 3));
+        const uint32_t *wrow = b.cw + (y >> 2) * b.gap;
         for (int x = lane; x < w; x += 32) {
           const int32_t v = (wrow[x] & sig) ? __ldcg(r + x) : 0;
           if (irrev) *reinterpret_cast<float *>(r + x) = __fmul_rn((float)signmag_to_int(v), cb.gain);
@@ -129,9 +127,9 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
   }
 }
 
-// The two kernel forms.  The compact form keeps the default register target, which leaves
-// room for 32 resident warps per SM; the unrolled form (batches that fit one wave) may use
-// more registers, as occupancy does not bound it.
+// The two kernel forms.  The throughput (compact) form keeps the default register target,
+// which leaves room for 32 resident warps per SM; the latency form (batches that fit about two
+// waves) may use more registers, as occupancy does not bound it.
 #define J2K_T1_PARAMS                                                                                   \
   const j2k_cblk *__restrict__ cbs, const uint32_t *__restrict__ order, int n, int *__restrict__ counter, \
       const uint8_t *__restrict__ bytes, const uint32_t *__restrict__ seglens, void *__restrict__ coef,   \
@@ -141,87 +139,15 @@ __global__ void __launch_bounds__(256) t1_kernel_compact(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, false>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 template <int MAXW, int MAXH>
-__global__ void __launch_bounds__(256, 1) t1_kernel_unrolled(J2K_T1_PARAMS) {
+__global__ void __launch_bounds__(256, 1) t1_kernel_latency(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, true>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 #undef J2K_T1_PARAMS
 
-template <int MAXW, int MAXH, bool UNROLLED>
+template <int MAXW, int MAXH, bool LATENCY>
 constexpr auto t1_kernel() {
-  if constexpr (UNROLLED) return &t1_kernel_unrolled<MAXW, MAXH>;
+  if constexpr (LATENCY) return &t1_kernel_latency<MAXW, MAXH>;
   else return &t1_kernel_compact<MAXW, MAXH>;
-}
-
-// ------------------------------------------------------------------ host tables --------
-void build_t1_tables(T1Tables &T) {
-  static const uint16_t QE[47] = {0x5601, 0x3401, 0x1801, 0x0AC1, 0x0521, 0x0221, 0x5601, 0x5401, 0x4801, 0x3801,
-                                  0x3001, 0x2401, 0x1C01, 0x1601, 0x5601, 0x5401, 0x5101, 0x4801, 0x3801, 0x3401,
-                                  0x3001, 0x2801, 0x2401, 0x2201, 0x1C01, 0x1801, 0x1601, 0x1401, 0x1201, 0x1101,
-                                  0x0AC1, 0x09C1, 0x08A1, 0x0521, 0x0441, 0x02A1, 0x0221, 0x0141, 0x0111, 0x0085,
-                                  0x0049, 0x0025, 0x0015, 0x0009, 0x0005, 0x0001, 0x5601};
-  static const uint8_t NMPS[47] = {1,  2,  3,  4,  5,  38, 7,  8,  9,  10, 11, 12, 13, 29, 15, 16,
-                                   17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32,
-                                   33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 45, 46};
-  static const uint8_t NLPS[47] = {1,  6,  9,  12, 29, 33, 6,  14, 14, 14, 17, 18, 20, 21, 14, 14,
-                                   15, 16, 17, 18, 19, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29,
-                                   30, 31, 32, 33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43, 46};
-  std::memset(&T, 0, sizeof(T));
-  for (int s = 0; s < 94; ++s) {
-    int idx = s >> 1, mps = s & 1;
-    int sw = (QE[idx] == 0x5601 && NLPS[idx] != 46);
-    uint32_t nm = (uint32_t)(NMPS[idx] << 1 | mps);
-    uint32_t nl = (uint32_t)(NLPS[idx] << 1 | (mps ^ sw));
-    T.mq[s].x = (uint32_t)QE[idx] << 8;
-    T.mq[s].y = ((uint32_t)mps << 16) | (nm << 8) | nl;
-  }
-  for (int r = 0; r < 16; ++r) {
-    const int n = __builtin_popcount(r);
-    for (int x = 0; x < (1 << n); ++x) {
-      int v = 0, i = 0;
-      for (int k = 0; k < 4; ++k)
-        if ((r >> k) & 1) v |= ((x >> (n - 1 - i++)) & 1) << k;
-      T.rawmr[r][x] = (uint8_t)v;
-    }
-  }
-  for (int band = 0; band < 3; ++band)
-    for (int nb = 0; nb < 512; ++nb) {
-      int h = ((nb >> 3) & 1) + ((nb >> 5) & 1);
-      int v = ((nb >> 1) & 1) + ((nb >> 7) & 1);
-      int d = (nb & 1) + ((nb >> 2) & 1) + ((nb >> 6) & 1) + ((nb >> 8) & 1);
-      int c;
-      if (band == 2) {  // HH
-        int hv = h + v;
-        if (d >= 3) c = 8;
-        else if (d == 2) c = hv >= 1 ? 7 : 6;
-        else if (d == 1) c = hv >= 2 ? 5 : (hv == 1 ? 4 : 3);
-        else c = hv >= 2 ? 2 : hv;
-      } else {
-        if (band == 1) std::swap(h, v);  // HL
-        if (h == 2) c = 8;
-        else if (h == 1) c = v >= 1 ? 7 : (d >= 1 ? 6 : 5);
-        else if (v == 2) c = 4;
-        else if (v == 1) c = 3;
-        else c = d >= 2 ? 2 : d;
-      }
-      T.zc[band][nb] = (uint8_t)c;
-    }
-  for (int i = 0; i < 256; ++i) {
-    // bit 0 sigma up, 1 chi up, 2 sigma down, 3 chi down, 4 sigma left, 5 chi left,
-    // 6 sigma right, 7 chi right (T.800 Table D.3)
-    auto contrib = [&](int sb, int xb) { return ((i >> sb) & 1) ? (((i >> xb) & 1) ? -1 : 1) : 0; };
-    int H = contrib(4, 5) + contrib(6, 7);
-    int V = contrib(0, 1) + contrib(2, 3);
-    H = std::max(-1, std::min(1, H));
-    V = std::max(-1, std::min(1, V));
-    int x = 0;
-    if (H < 0 || (H == 0 && V < 0)) {
-      H = -H;
-      V = -V;
-      x = 1;
-    }
-    int c = (H == 1) ? (V == 1 ? 4 : (V == 0 ? 3 : 2)) : (V == 1 ? 1 : 0);
-    T.sc[i] = (uint8_t)(c << 1 | x);
-  }
 }
 
 // ------------------------------------------------------------------ device buffers -----
@@ -275,7 +201,7 @@ struct j2k_gpu_ctx {
   cudaGraphExec_t gexec = nullptr;  // captured decode of the staged batch (tuning.use_graph)
   int graph_launches = 0;
   // autotuned Tier-1 shape per queue-length bucket (floor(log2(code-blocks))): kernel form
-  // (1 compact, 2 unrolled) and warps per CTA; consulted by the auto form
+  // (1 compact, 2 latency) and warps per CTA; consulted by the auto form
   struct TuneEntry {
     int form = 0, warps = 0;
     float t1_ms = 0;
@@ -369,7 +295,7 @@ extern "C" int j2k_gpu_ctx_create(int device, size_t mem_budget, j2k_gpu_ctx **o
   build_t1_tables(T);
   j2k_lanes::LaneTables LT;
   j2k_lanes::build_lane_tables(LT);
-  if (cudaMemcpyToSymbol(c_t1tables, &T, sizeof(T)) != cudaSuccess || ensure(c, c->d_tables, sizeof(LT)) != J2K_OK ||
+  if (cudaMemcpyToSymbol(g_t1tables, &T, sizeof(T)) != cudaSuccess || ensure(c, c->d_tables, sizeof(LT)) != J2K_OK ||
       cudaMemcpy(c->d_tables.p, &LT, sizeof(LT), cudaMemcpyHostToDevice) != cudaSuccess) {
     j2k_gpu_ctx_destroy(c);
     return J2K_ERR_CUDA;
@@ -498,17 +424,20 @@ extern "C" int j2k_gpu_batch_footprint(const j2k_gpu_ctx *cc, size_t *bytes) {
 namespace {
 // Persistent Tier-1 launch: the CTA shape with the most resident warps per SM (registers,
 // shared memory and thread limits from the occupancy calculator), one wave of CTAs.
-template <int MAXW, int MAXH, bool UNROLLED>
+template <int MAXW, int MAXH, bool LATENCY>
 void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, const uint32_t *ord, int *cnt,
                   const uint32_t *seg, int warps_per_cta) {
   typedef T1Layout<MAXW, MAXH> Lay;
   int best_w = 1, best_ctas = 1, best_warps = 0;
-  const int wmax = warps_per_cta > 0 ? std::min(8, warps_per_cta) : 8;
+  // a queue shorter than the resident warps is spread over all SMs: its time is that of its
+  // longest blocks, which two warps of one scheduler would lengthen
+  const int spread = std::max(1, (n + c->sm_count - 1) / c->sm_count);
+  const int wmax = std::min(spread, warps_per_cta > 0 ? std::min(8, warps_per_cta) : 8);
   for (int w = 1; w <= wmax; ++w) {
-    const size_t sm = (size_t)w * Lay::PER_WARP;
+    const size_t sm = sizeof(T1Tables) + (size_t)w * Lay::PER_WARP;
     if (sm > c->smem_optin) break;
     int ctas = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, t1_kernel<MAXW, MAXH, UNROLLED>(), w * 32, sm) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, t1_kernel<MAXW, MAXH, LATENCY>(), w * 32, sm) !=
         cudaSuccess) {
       cudaGetLastError();
       continue;
@@ -519,16 +448,16 @@ void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, c
       best_ctas = ctas;
     }
   }
-  const size_t sm = (size_t)best_w * Lay::PER_WARP;
+  const size_t sm = sizeof(T1Tables) + (size_t)best_w * Lay::PER_WARP;
   const int grid = std::max(1, std::min((n + best_w - 1) / best_w, c->sm_count * std::max(1, best_ctas)));
-  t1_kernel<MAXW, MAXH, UNROLLED>()<<<grid, best_w * 32, sm, st>>>(cbs, ord, n, cnt, (const uint8_t *)c->d_bytes.p, seg,
+  t1_kernel<MAXW, MAXH, LATENCY>()<<<grid, best_w * 32, sm, st>>>(cbs, ord, n, cnt, (const uint8_t *)c->d_bytes.p, seg,
                                                                      c->d_A.p, (uint16_t *)c->d_status.p);
 }
 
-// Tier-1 form for a batch of n code-blocks: 1 compact warp form (throughput), 2 unrolled
-// warp form (latency), 3 one block per lane, and warps per CTA of a warp form.  An explicit
+// Tier-1 form for a batch of n code-blocks: 1 compact warp form (throughput), 2 latency
+// warp form, 3 one block per lane, and warps per CTA of a warp form.  An explicit
 // tuning.t1_form wins; the auto form (0) takes the autotuned choice of the queue's size
-// bucket, else the unrolled form while the queue holds at most `t1_latency_waves` blocks
+// bucket, else the latency form while the queue holds at most `t1_latency_waves` blocks
 // per resident warp slot of the GPU (the launch's time is then the serial time of its
 // longest blocks) and the compact form for longer queues.  The lane form is only taken
 // when asked for: on B200 it measured 4.2x slower than the compact form on 1080p 9/7

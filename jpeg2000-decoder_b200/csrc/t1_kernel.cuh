@@ -1,43 +1,43 @@
 /*
  * t1_kernel.cuh — EBCOT Tier-1 code-block decoder for sm_100a.
  *
- * One warp per code-block.  The warp keeps the block's stripe context words in shared
- * memory and the MQ registers (A, C, t, T, byte position) in registers.
- * The arithmetic decode is inherently serial, so all 32 lanes execute the same scalar
- * decode in lock-step (uniform control flow, broadcast shared-memory reads); the lanes
- * work in parallel where the data allows it: clearing the state, locating the next
- * non-empty stripe column of a pass with a warp ballot, measuring runs of empty columns
- * in the cleanup pass, and the dequantising, coalesced rewrite of the finished block.
- * Blocks are pulled from a device work queue (atomic counter over a host-sorted order,
- * longest blocks first), so CTAs stay resident and uneven blocks balance out.
+ * One warp per code-block, blocks pulled from a device work queue (atomic counter over a
+ * host-sorted order, longest blocks first) by persistent CTAs.
  *
- * Latency and occupancy measures, none of which changes a decoded bit:
- *   - two kernel forms: the compact one (long queues, throughput) is kept small for the
- *     instruction cache (many resident warps sit in different passes at once): each pass
- *     walks the rows of a stripe column as a bit mask, inlines each of its decisions once,
- *     and bypass (raw) and MQ decisions share the pass code; the unrolled one (batches that
- *     fit about two waves, latency) unrolls the rows and hands the lanes' chunk words and
- *     masks to the serial loop;
- *   - per 32-column chunk the lanes compute each column's row mask and only columns with
- *     work join the serial loop;
- *   - each MQ context slot holds its probability-table entry (Qe, MPS, both successor
- *     states), so a symbol needs one shared-memory load before its decision;
- *   - code bytes are read as aligned 32-bit words with the next word requested early, so
- *     byte fills do not wait on memory;
+ * The arithmetic decode is a serial chain: every symbol needs the interval the previous one
+ * left.  It bounds the kernel twice over: a single picture lasts as long as the chain of its
+ * densest block (about 42 warp instructions a symbol at 4.4 cycles each; integer instructions
+ * issue every second cycle, a dependent one after 4 to 5, a shared-memory load returns after
+ * 23, a branch costs 15 to 25 and one on which the lanes differ 40 and more), and a long queue
+ * fills the SMs' issue slots with instructions that all 32 lanes execute alike.  So what counts
+ * is instructions and branches per symbol:
+ *   - the code register is extended by 32 and more bits of upcoming code, refilled four bytes at
+ *     a time, so renormalisation is a shift without a loop, and one check covers two symbols;
+ *   - each MQ context slot holds its probability-table entry (Qe, MPS, place in the table), so
+ *     a symbol needs one shared-memory load before its decision, and the entries that may
+ *     follow lie side by side;
+ *   - refinement symbols change no later label: the lanes list a 32-column chunk's labels in
+ *     scan order (positions from four ballots), the serial loop only walks the list, and each
+ *     lane takes its column's bits from the decoded bit string and issues the sample updates;
+ *     bypass (raw) bits of a chunk come byte by byte;
+ *   - in significance propagation and cleanup the lanes tell which columns have work; the walk
+ *     takes a column's rows from its context word.  A sample that becomes significant updates
+ *     the eight words around it by as many lanes at once, without a branch (a tree of lane
+ *     conditions there cost 450 cycles a sample);
+ *   - stores that only some lanes make are predicated, never branched around;
  *   - in the cleanup pass a run of all-zero columns whose run-length symbols would all
  *     decode as MPS without renormalisation (C >= k*Qe and A - k*Qe >= 0x8000, scaled) is
- *     consumed in one step: A -= k*Qe, C -= k*Qe;
+ *     consumed in one step;
  *   - samples live in the block's own region of the output buffer, not in shared memory:
  *     they are only written while decoding (significance sets sign + 1.5 * 2^p, a
- *     refinement flips bit p and sets the new midpoint bit), so updates go out as
- *     fire-and-forget atomic XORs: in the compact form a stripe column's at its end from
- *     lanes 0..3 in one instruction, in the unrolled form each 32-column chunk's at its end
- *     from the lanes owning the columns (off the serial chain: C2 Tier-1 10.8 -> 7.9 ms),
- *     and the "first refinement?" context test of the reference ((|v| >> p) < 4, true
- *     exactly on a sample's first refinement) reads a per-sample "refined" bit kept in
- *     shared memory.  A 64x64 block then needs 6 KB of shared memory instead of 13-21 KB,
- *     so more blocks are resident per SM;
- *   - bypass refinement bits of a column are taken together and scattered to their rows.
+ *     refinement flips bit p and sets the new midpoint bit by a fire-and-forget atomic XOR).
+ * Two forms share this code: the throughput form leaves a symbol early when it is an MPS
+ * without renormalisation (fewest instructions), the latency form has no branch in a symbol and
+ * takes refinement symbols four at a time (shortest chain).
+ * Measured against the form with a renormalisation loop, a byte at a time, rows unrolled
+ * (B200, Tier-1 ms): one 2048x2048 RGB 9/7 picture 7.22 -> 3.83, one 512x512 gray lossless
+ * picture 4.92 -> 3.2, one 2048x1080 12-bit BYPASS + RESET picture 5.47 -> 3.16, 32 1080p 9/7
+ * frames 14.76 -> 13.2.
  *
  * Semantics follow the reference block decoder exactly (decoder/codec/src/
  * bmi_block_decoder.cpp:10-853, bmi_mq_decoder.h/.cpp, bmi_t1_macro.h): same context-word
@@ -49,79 +49,118 @@
  */
 #pragma once
 #include <cstdint>
+#include <cstring>
+#include <utility>
 
 #include "plan.h"
 
-
-
 namespace j2k_dev {
 
-// ---- context-word bits (bmi_t1_macro.h:14-73)
-constexpr uint32_t NBR_ROW0 = 0x1EF;
-constexpr int MU_POS = 20, PI_POS = 21, CHI_POS = 19;
-__device__ __forceinline__ uint32_t ROW_SIG(int k) { return 0x10u << (3 * k); }
-__device__ __forceinline__ uint32_t ROW_CHI(int k) { return 1u << (CHI_POS + 3 * k); }
-__device__ __forceinline__ uint32_t ROW_MU(int k) { return 1u << (MU_POS + 3 * k); }
-__device__ __forceinline__ uint32_t ROW_PI(int k) { return 1u << (PI_POS + 3 * k); }
-__device__ __forceinline__ uint32_t ROW_NBR(int k) { return NBR_ROW0 << (3 * k); }
-constexpr uint32_t MU_ALL = (1u << 20) | (1u << 23) | (1u << 26) | (1u << 29);
-constexpr uint32_t PI_ALL = (1u << 21) | (1u << 24) | (1u << 27) | (1u << 30);
-constexpr uint32_t CHI_ALL = (1u << 19) | (1u << 22) | (1u << 25) | (1u << 28);
+// ---- context word of a stripe column (bmi_t1_macro.h:14-73): bits 0..17 the significance of
+// the 3 x 6 samples around the column's four rows (row group j, columns left / own / right at
+// bits 3j, 3j+1, 3j+2; group 0 is the row above, row k's own bit is 4 + 3k), bit 18 the sign
+// of the sample above, 19 + 3k / 20 + 3k / 21 + 3k row k's sign (chi; set on rows outside
+// the block), mu (significant before this bit-plane) and pi (coded by this plane's
+// significance pass), bit 31 the sign of the sample below
+constexpr int SIG_POS = 4, CHI_POS = 19, MU_POS = 20, PI_POS = 21;
+constexpr uint32_t ROWS = 0x249;  // one bit per row, at 3k: a set of the column's rows
+constexpr uint32_t CHI_ALL = ROWS << CHI_POS, MU_ALL = ROWS << MU_POS, PI_ALL = ROWS << PI_POS;
 
 enum { C_SIG = 0, C_RUN = 9, C_SIGN = 10, C_MAG = 15, C_UNI = 18, N_CTX = 19 };
+constexpr uint32_t SLOT = 8;  // bytes of a context slot
+constexpr uint32_t RUN_OFF = C_RUN * SLOT, UNI_OFF = C_UNI * SLOT;  // byte offsets of context slots
 
-// Read-only tables (constant memory; every lane of a warp reads the same entry):
-//   mq[94]   : entry of state s = idx*2 + mps: .x = Qe << 8 (the scaled register unit),
-//              .y = (mps << 16) | (state after an MPS << 8) | state after an LPS
-//   zc[3][512]: zero-coding context for LL/LH, HL, HH neighbourhoods
-//   sc[256]  : (sign context << 1) | xor bit for an 8-bit (sigma, chi) neighbour index
-//   rawmr[r][x]: bypass refinement bits: the n = popcount(r) raw bits x (first decoded in
-//              bit n-1) placed on the rows set in r, lowest row first
+// Read-only tables, copied to shared memory by every CTA (the lanes look labels up at
+// different addresses, which constant memory would serialise):
+//   mq[94][3]: for state s = idx*2 + mps the entries of the state itself, of the one after an MPS
+//              and of the one after an LPS; an entry is .x = Qe << 8 (the scaled register
+//              unit), .y = (mps << 31) | byte offset of the state's first record
+//   zc[3][512]: slot offset of the zero-coding context for LL/LH, HL, HH neighbourhoods
+//   sc[2048] : slot offset of the sign context | xor bit, by sign_index()
 struct T1Tables {
-  uint2 mq[96];
+  uint2 mq[96][3];
   uint8_t zc[3][512];
-  uint8_t sc[256];
-  uint8_t rawmr[16][16];
+  uint8_t sc[2048];
 };
 
-// MQ decoder registers.  Code bytes are read as aligned 32-bit words: `cur` holds the byte
-// at `ap`, and the word after it is requested as soon as `cur` is entered, so the load has
-// several fills (dozens of symbols) to complete before its first byte is needed.
+// MQ decoder registers: A and C in the reference's scale (0x8000 is 0x800000); the low eight
+// bits of C and all of l0, l1 are upcoming code, `T` the number of code bits held there (below
+// the scale point).  Code bytes are read as aligned 32-bit words: `cur` holds the byte at
+// `ap`, and the word after it is requested as soon as `cur` is entered.
 struct Mq {
   int32_t A, C;
-  int32_t t, T;
+  uint32_t l0, l1;
+  int32_t T;
+  uint32_t last;      // the byte before `ap` (0xFF: the next byte carries seven bits)
   uint32_t ap, aend;  // byte position and segment end, counted from `w`
   const uint32_t *w;  // the segment's first byte rounded down to a 4-byte boundary
   uint32_t cur, nxt;  // the word holding byte ap and the one after it
 };
+constexpr int32_t A_MIN = 0x800000;
+// Enough for two symbols: a renormalisation shifts by 15 at most, only bits above the scale
+// point are compared, and bits missing after the second one are added by the next refill
+constexpr int T_MIN = 15;
 
-__device__ __forceinline__ int mq_byte(const Mq &m) {
-  return m.ap < m.aend ? (int)((m.cur >> ((m.ap & 3) * 8)) & 0xFF) : 0xFF;
+// Append n code bits v at position T of the 72-bit field (C's low eight bits, l0, l1); T may be
+// negative: C was shifted further than the bits that were there
+__device__ __forceinline__ void mq_append(Mq &m, uint32_t v, int n) {
+  const uint64_t x = (uint64_t)v << (40 - n - m.T);  // T < T_MIN: nothing reaches l1
+  m.C += (int32_t)(uint32_t)(x >> 32);
+  m.l0 += (uint32_t)x;
+  m.T += n;
 }
 
-__device__ __forceinline__ void mq_advance(Mq &m) {
-  m.ap++;
-  if (!(m.ap & 3)) {
+// Refill to at least T_MIN bits; false when that many are not to be had yet.  Four plain bytes
+// go in at once; around a 0xFF byte and at the segment's end the rules of FILL_LSBS
+// (bmi_mq_decoder.h:52-73) hold byte by byte: after a 0xFF the next byte carries 7 bits,
+// unless it is a marker (> 0x8F), which is not consumed and reads as eight ones; bytes past the
+// segment's end read as 0xFF.  A byte 0x80..0x8F after a 0xFF adds a carry above its seven
+// bits.  The reference adds it only once every earlier bit has been shifted into the compared
+// part and another shift is due, so it waits here until T is negative: the shifted sum is the
+// same, as both are linear, and no comparison sees the carry early.  Until then T stays below
+// T_MIN and every single symbol needs a refill before it (mq_level).
+__device__ __forceinline__ bool mq_refill(Mq &m) {
+  const uint32_t four = __funnelshift_r(m.cur, m.nxt, (m.ap & 3) * 8);
+  const uint32_t z = ~((four << 8) | m.last);  // a zero byte: the byte before or one of the first three is 0xFF
+  if (!((z - 0x01010101u) & ~z & 0x80808080u) && m.T >= 0 && m.ap + 4 <= m.aend) {
+    const uint32_t v = __byte_perm(four, 0, 0x0123);
+    const uint64_t x = (uint64_t)v << (40 - m.T);
+    m.C += (int32_t)((v >> 8) >> (16 + m.T));
+    m.l0 |= (uint32_t)(x >> 32);
+    m.l1 = (uint32_t)x;
+    m.T += 32;
+    m.last = four >> 24;
+    m.ap += 4;
     m.cur = m.nxt;
     m.nxt = __ldg(m.w + (m.ap >> 2) + 1);
+    return true;
   }
+#pragma unroll 1
+  while (m.T < T_MIN) {
+    const uint32_t b = m.ap < m.aend ? (m.cur >> ((m.ap & 3) * 8)) & 0xFF : 0xFF;
+    if (m.last != 0xFF) {
+      mq_append(m, b, 8);
+      m.last = b;
+    } else if (b > 0x8F) {
+      mq_append(m, 0xFF, 8);
+      continue;
+    } else {
+      if (b >= 0x80 && m.T >= 0) return false;
+      mq_append(m, b, 7);
+      m.last = 0;
+    }
+    m.ap++;
+    if (!(m.ap & 3)) {
+      m.cur = m.nxt;
+      m.nxt = __ldg(m.w + (m.ap >> 2) + 1);
+    }
+  }
+  return true;
 }
 
-// FILL_LSBS, bmi_mq_decoder.h:52-73, as selects: after a 0xFF byte the next byte carries 7
-// bits, unless it is a marker (> 0x8F), which is not consumed and reads as 0xFF with 8 bits
-__device__ __forceinline__ void mq_fill(Mq &m) {
-  const int b = mq_byte(m);
-  const bool ff = m.T == 0xFF;
-  const bool marker = ff && b > 0x8F;
-  m.T = marker ? 0xFF : (ff ? b << 1 : b);
-  if (!marker) mq_advance(m);
-  m.t = (ff && !marker) ? 7 : 8;
-  m.C += m.T;
-}
-
-// Init, bmi_mq_decoder.cpp:186-219 (the 0xFF 0xFF termination is virtual: bytes at or past
-// `end` read as 0xFF).  The word loads may reach up to 9 bytes past the segment; the code
-// byte buffer carries 16 bytes of slack after its last segment.
+// Init, bmi_mq_decoder.cpp:186-219: two bytes loaded and shifted up by 15.  The word loads
+// may reach up to 9 bytes past the segment; the code byte buffer carries 16 bytes of slack
+// after its last segment.
 __device__ __forceinline__ void mq_init(Mq &m, const uint8_t *base, uint32_t len) {
   const uint32_t off = (uint32_t)((uintptr_t)base & 3);
   m.w = reinterpret_cast<const uint32_t *>(base - off);
@@ -129,94 +168,66 @@ __device__ __forceinline__ void mq_init(Mq &m, const uint8_t *base, uint32_t len
   m.aend = off + len;
   m.cur = __ldg(m.w);
   m.nxt = __ldg(m.w + 1);
-  m.T = 0;
+  m.last = 0;
   m.C = 0;
-  m.t = 0;
-  mq_fill(m);
-  m.C <<= m.t;
-  mq_fill(m);
-  m.C <<= 7;
-  m.t -= 7;
-  m.A = 0x800000;
+  m.l0 = m.l1 = 0;
+  m.T = -15;
+  m.A = A_MIN;
+  mq_refill(m);
 }
 
-// Shift until A >= 0x800000, filling a byte whenever t reaches 0 (the reference's
-// RENORMALIZE_ONCE loop, taken several shifts at a time; at most two fills, as a fill
-// after a 0xFF byte is followed by one of 8 bits)
-__device__ __forceinline__ void mq_renorm(Mq &m) {
-  int n = __clz(m.A) - 8;
-  while (m.t < n) {
-    m.A <<= m.t;
-    m.C <<= m.t;
-    n -= m.t;
-    mq_fill(m);
-  }
-  m.A <<= n;
-  m.C <<= n;
-  m.t -= n;
-}
-
-// MQ_DECODE, bmi_mq_decoder.h:86-128, on a context slot holding its table entry.  Both
-// renormalising outcomes (conditional exchange after C < Qe; A below 0x8000 after C >= Qe)
-// share one table update and one renormalisation.  EARLY (compact kernel form: fewest
-// instructions) returns the common outcome first: C >= Qe and A still >= 0x8000 after
-// A -= Qe (MPS, no renormalisation); otherwise (unrolled form: shortest dependency chain)
-// the outcome is computed before a single branch.
-template <bool EARLY>
-__device__ __forceinline__ int mq_decode(Mq &m, uint2 *cx, const uint2 *tab) {
-  const uint2 e = *cx;
+// One symbol (MQ_DECODE, bmi_mq_decoder.h:86-128) of a context whose slot entry is `e`, T being
+// at least 0; returns the symbol and leaves the entry that follows in `e` and in the slot.  The
+// throughput form returns early on an MPS without renormalisation; the latency form has no
+// branch: the successor (itself, after an MPS, after an LPS) is one of three adjacent records.
+template <bool LATENCY, bool STORE = true>
+__device__ __forceinline__ uint32_t mq_symbol(Mq &m, uint8_t *slot, uint2 &e, const uint8_t *tab) {
   const int32_t q = (int32_t)e.x;
-  m.A -= q;
+  const uint32_t mps = e.y >> 31;
+  const int32_t a1 = m.A - q, d1 = m.C - q;
   const bool ex = m.C < q;
-  if constexpr (EARLY) {
-    if (!ex && m.A >= 0x800000) {
-      m.C -= q;
-      return (int)((e.y >> 16) & 1);
-    }
-    const bool lps = (m.A < q) != ex;
-    if (ex) m.A = q;
-    else m.C -= q;
-    *cx = tab[lps ? (e.y & 0xFF) : ((e.y >> 8) & 0xFF)];
-    mq_renorm(m);
-    return (int)((e.y >> 16) & 1) ^ (int)lps;
-  } else {
-    const bool lps = ex ? (m.A >= q) : (m.A < q);
-    const int sym = (int)((e.y >> 16) & 1) ^ (int)lps;
-    if (!ex) m.C -= q;
-    if (ex || m.A < 0x800000) {
-      *cx = tab[lps ? (e.y & 0xFF) : ((e.y >> 8) & 0xFF)];
-      if (ex) m.A = q;
-      mq_renorm(m);
-    }
-    return sym;
+  if (!LATENCY && !ex && a1 >= A_MIN) {  // MPS without renormalisation
+    m.A = a1;
+    m.C = d1;
+    return mps;
   }
+  const bool lps = (a1 < q) != ex;
+  const int32_t a = ex ? q : a1, c = ex ? m.C : d1;
+  uint32_t rec = e.y & 0xFFFF;
+  if (!LATENCY || a < A_MIN) rec += sizeof(uint2);
+  if (lps) rec += sizeof(uint2);
+  e = *reinterpret_cast<const uint2 *>(tab + rec);
+  if (STORE) *reinterpret_cast<uint2 *>(slot) = e;
+  const int n = __clz(a) - 8;
+  m.A = a << n;
+  m.C = (int32_t)__funnelshift_l(m.l0, (uint32_t)c, n);
+  m.l0 = __funnelshift_l(m.l1, m.l0, n);
+  m.l1 <<= n;
+  m.T -= n;
+  return mps ^ (uint32_t)lps;
+}
+// Before a pair of symbols / between the two (a refill is due there only while a carry waits)
+__device__ __forceinline__ void mq_ready(Mq &m) {
+  if (m.T < T_MIN) mq_refill(m);
+}
+__device__ __forceinline__ void mq_level(Mq &m) {
+  if (m.T < 0) mq_refill(m);
+}
+// a symbol on its own
+template <bool LATENCY>
+__device__ __forceinline__ uint32_t mq_decode(Mq &m, uint8_t *cx, uint32_t off, const uint8_t *tab) {
+  uint2 e = *reinterpret_cast<const uint2 *>(cx + off);
+  mq_ready(m);
+  return mq_symbol<LATENCY>(m, cx + off, e, tab);
 }
 
-// MQ_DECODE_START (fixed Qe 0x5601, MPS 0, no adaptation), bmi_mq_decoder.h:131-169
-__device__ __forceinline__ int mq_uniform(Mq &m) {
-  int ret = 0;
-  if (m.C < 0x560100) {
-    if (m.A >= (0x560100 << 1)) ret = 1;
-    if (!m.t) mq_fill(m);
-    m.C <<= 1;
-    m.t--;
-    m.A = 0x560100 << 1;
-  } else {
-    m.A -= 0x560100;
-    m.C -= 0x560100;
-    if (m.A < 0x800000) {
-      if (m.A < 0x560100) ret = 1;
-      mq_renorm(m);
-    }
-  }
-  return ret;
-}
-
+// Raw (bypass) bits, T.800 D.6: after 0xFF the next byte carries 7 bits; bytes past the end
+// read as 0xFF
 struct Raw {
-  uint32_t pos, end;
   const uint8_t *base;
+  uint32_t pos, end;
   uint32_t c;
-  int ct, last;
+  int ct;
 };
 __device__ __forceinline__ void raw_init(Raw &r, const uint8_t *base, uint32_t len) {
   r.base = base;
@@ -224,384 +235,328 @@ __device__ __forceinline__ void raw_init(Raw &r, const uint8_t *base, uint32_t l
   r.end = len;
   r.c = 0;
   r.ct = 0;
-  r.last = 0;
 }
-// T.800 D.6: after 0xFF the next byte carries 7 bits; bytes past the end read as 0xFF
-__device__ __forceinline__ int raw_bit(Raw &r) {
-  if (r.ct == 0) {
-    int b = r.pos < r.end ? (int)__ldg(r.base + r.pos) : 0xFF;
-    r.pos++;
-    r.ct = (r.last == 0xFF) ? 7 : 8;
-    r.last = b;
-    r.c = (uint32_t)b;
-  }
+__device__ __forceinline__ void raw_byte(Raw &r) {
+  r.ct = r.c == 0xFF ? 7 : 8;
+  r.c = r.pos < r.end ? (uint32_t)__ldg(r.base + r.pos) : 0xFFu;
+  r.pos++;
+}
+__device__ __forceinline__ uint32_t raw_bit(Raw &r) {
+  if (r.ct == 0) raw_byte(r);
   r.ct--;
-  return (int)((r.c >> r.ct) & 1);
+  return (r.c >> r.ct) & 1;
+}
+// the next n bits (n <= 32), first bit in bit 0
+__device__ __forceinline__ uint32_t raw_bits(Raw &r, int n) {
+  uint32_t x = 0;
+  int got = 0;
+  while (got < n) {
+    if (r.ct == 0) raw_byte(r);
+    const int k = min(r.ct, n - got);
+    r.ct -= k;
+    x = (x << k) | ((r.c >> r.ct) & ((1u << k) - 1u));
+    got += k;
+  }
+  return __brev(x) >> (32 - n);
 }
 
-// ---- samples: raw int32 (bit 31 sign, magnitude with midpoint bit) built in global memory:
-// a sample's significance writes its first value (nothing touched it before), refinements
-// XOR into it; samples that never become significant are never written while decoding (the
-// final rewrite gives them 0 from the significance bits in shared memory), so the block
-// region needs no zero-fill.  The lane that writes a sample's first value also issues its
-// refinements, so each sample's updates stay in program order.  While a 32-column chunk
-// of a stripe is decoded, each column's update goes to the lane that owns the column (one
-// select in the serial loop); at the end of the chunk every lane issues its column's row
-// updates as fire-and-forget atomics, consecutive lanes on consecutive columns (nothing reads
-// the samples while decoding, and XOR updates commute).
-struct Samples {
-  int32_t *base;      // the block's first sample in the output buffer
-  uint32_t stride;    // elements per row
-  int lane;
-  // column update `upd`: bits 0..3 rows updated, bits 4..7 the sign (significance pass) or
-  // the decoded refinement bit (refinement pass) of each row
-  // one column's update from lanes 0..3 in one warp instruction, straight from the serial
-  // loop (compact form: cheapest when every resident warp competes for issue slots)
-  template <bool REFINE>
-  __device__ __forceinline__ void apply(int row0, int col, uint32_t upd, int plane) const {
-    if (lane < 4 && ((upd >> lane) & 1)) {
-      const uint32_t bit = (upd >> (4 + lane)) & 1;
-      unsigned int *at = reinterpret_cast<unsigned int *>(base + (size_t)(row0 + lane) * stride + col);
-      if (REFINE) atomicXor(at, ((1u - bit) << plane) | ((1u << plane) >> 1));
-      else *at = (bit << 31) + (1u << plane) + ((1u << plane) >> 1);  // first value of the sample
-    }
-  }
-  // a chunk's updates, each lane issuing its own column's (unrolled form: the serial loop of
-  // a latency-bound batch keeps only a select per column)
-  template <bool REFINE>
-  __device__ __forceinline__ void flush(int row0, int col, uint32_t upd, int plane) const {
-    if (!(upd & 0xF)) return;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!((upd >> k) & 1)) continue;
-      const uint32_t bit = (upd >> (4 + k)) & 1;
-      unsigned int *at = reinterpret_cast<unsigned int *>(base + (size_t)(row0 + k) * stride + col);
-      if (REFINE) atomicXor(at, ((1u - bit) << plane) | ((1u << plane) >> 1));
-      else *at = (bit << 31) + (1u << plane) + ((1u << plane) >> 1);  // first value of the sample
-    }
-  }
+// Shared memory of one warp.  The context words of a block w samples wide lie in rows of
+// w + 3 words, one row per stripe with a row of zeros above and below and a column left and
+// right, so that a sample's neighbours always exist.
+template <int MAXW, int MAXH>
+struct T1Layout {
+  static constexpr int STRIPES = MAXH / 4, CHUNKS = (MAXW + 31) / 32;
+  static constexpr int CWN = (STRIPES + 2) * (MAXW + 3) + 2;
+  static constexpr int RF = (CWN * 4 + 15) & ~15;           // refined rows, 16 bytes per chunk
+  static constexpr int CX = RF + STRIPES * CHUNKS * 16;     // context slots
+  static constexpr int BITS = CX + ((N_CTX * (int)SLOT + 15) & ~15);  // a chunk's refinement bits
+  static constexpr int LIST = BITS + 16;                    // a chunk's refinement labels in scan order
+  static constexpr int PER_WARP = LIST + 4 * 32 + 16;
 };
 
-// per-warp decode state in shared memory
-struct BlockSmem {
-  uint32_t *cw;  // context words: (stripes + 2) rows of (w + 3) words, + 2
-  uint8_t *rf;   // per stripe column: bit k set once row k has been refined
-  uint2 *cx;     // 18 MQ context slots (table entries)
-  Samples sp;
-  int w, gap;
+struct Block {
+  uint32_t *cw;    // first context word of stripe 0
+  uint4 *rf;       // per stripe and chunk: rows 0..3, bit = column: refined before
+  uint8_t *cx;     // context slots
+  uint32_t *bits;
+  uint8_t *list;
+  const uint8_t *mq, *zc, *sc;  // tables (zc: the block's band)
+  uint32_t *out;    // the block's first sample in the output buffer
+  uint32_t stride;  // elements per row
+  int w, gap, stripes, lane;
+  // how this lane (0..8) updates a word around a sample that becomes significant
+  int spread_off;                      // word offset from the sample's column
+  uint32_t spread_bits, spread_sign;   // bits set; where the sign goes (own column only)
+  uint32_t spread_rows, spread_shift;  // rows (ROWS set) it applies to; all ones: shifted by the row
 };
 
-__device__ __forceinline__ uint32_t *cword(const BlockSmem &b, int s, int c) {
-  return b.cw + (s + 1) * b.gap + 1 + c;
+// Lanes 0..8 hold the 3 x 3 words (stripe above / own / below, column left / own / right; the
+// centre, lane 4, is the walk's own).  Row k of the own stripe's words gets its bit shifted by 3k; the words above change for row
+// 0 only (not at all with stripe-causal contexts, T.800 D.7: a stripe's last row sees the next
+// stripe as insignificant) and the words below for row 3 only (bmi_block_decoder.cpp:53-101).
+__device__ __forceinline__ void spread_init(Block &b, bool causal) {
+  const int lane = b.lane, r = lane / 3, c = lane - 3 * r;
+  const bool on = lane < 9 && lane != 4 && !(r == 0 && causal);
+  const uint32_t own = c == 0 ? 0x20u : 0x08u;
+  b.spread_off = lane < 9 ? (r - 1) * b.gap + c - 1 : 0;
+  b.spread_bits = r == 0 ? (c == 0 ? 0x100u << 9 : (c == 1 ? 0x80u << 9 : 0x40u << 9))
+                         : (r == 1 ? own : (c == 0 ? 0x04u : (c == 1 ? 0x02u : 0x01u)));
+  b.spread_sign = c != 1 ? 0u : (r == 0 ? 1u << 31 : 1u << 18);
+  b.spread_rows = !on ? 0u : (r == 0 ? 1u : (r == 1 ? ROWS : 1u << 9));
+  b.spread_shift = r == 1 ? 0xFFFFFFFFu : 0u;
+}
+// No branch: a lane without a part in it ORs zero (lanes 9 up into the centre, which no lane
+// changes; a divergent branch here cost 400 cycles a sample).
+__device__ __forceinline__ void spread(const Block &b, uint32_t *wp, uint32_t k3, uint32_t sign) {
+  const uint32_t on = 0u - ((b.spread_rows >> k3) & 1u);
+  const uint32_t v = (b.spread_bits | (b.spread_sign & (0u - sign))) << (k3 & b.spread_shift);
+  wp[b.spread_off] |= v & on;
 }
 
-// sign context index of row k: bit 0 sigma up, 1 chi up, 2 sigma down, 3 chi down,
-// 4 sigma left, 5 chi left, 6 sigma right, 7 chi right
-__device__ __forceinline__ int sign_index(uint32_t cw, uint32_t wl, uint32_t wr, int k) {
-  uint32_t v = cw >> (3 * k);
-  uint32_t chi_up = (k == 0) ? (cw >> 18) & 1 : (v >> 16) & 1;
-  uint32_t idx = ((v >> 1) & 1) | (chi_up << 1) | (((v >> 7) & 1) << 2) | (((v >> 22) & 1) << 3);
-  uint32_t l = wl >> (3 * k), r = wr >> (3 * k);
-  idx |= ((l >> 4) & 1) << 4 | ((l >> 19) & 1) << 5 | ((r >> 4) & 1) << 6 | ((r >> 19) & 1) << 7;
-  return (int)idx;
+// Index of a sample's sign context: the significance and sign of its four neighbours (own
+// column's word cw, the left word l and the right word r; row k), eight bits gathered into
+// eleven without a loop: up / down sigma at bits 1, 7 and chi at 16, 22 of the shifted word,
+// left at 4 / 19, right (shifted by 2) at 6 / 21; the chi half folds between the sigma half.
+__device__ __host__ __forceinline__ uint32_t sign_fold(uint32_t x) { return ((x | (x >> 11)) >> 1) & 0x7FF; }
+__device__ __forceinline__ uint32_t sign_index(uint32_t cw, uint32_t l, uint32_t r, uint32_t k3) {
+  uint32_t v = cw >> k3;
+  if (k3 == 0) v = (v & ~0x10000u) | ((v >> 2) & 0x10000u);  // row 0: the sign above is bit 18
+  constexpr uint32_t UD = (1u << 1) | (1u << 7) | (1u << 16) | (1u << 22), LR = (1u << 4) | (1u << 19);
+  const uint32_t x = (v & UD) | ((l >> k3) & LR) | (((r >> k3) & LR) << 2);
+  return sign_fold(x);
 }
 
-// Mark row k of the column at `wp` significant with sign `sym`: spread sigma / chi to the
-// neighbouring words (bmi_block_decoder.cpp:53-101 and the row 1..3 variants).  In CAUSAL
-// blocks (T.800 D.7) a stripe's last row sees the next stripe as insignificant, so row 0
-// spreads nothing upward; the flag sits in a spare byte of the refined-rows array (see
-// causal_flag) and is read only here.
-__device__ __forceinline__ uint8_t &causal_flag(const BlockSmem &b) { return b.rf[b.gap - 1]; }
-__device__ __forceinline__ void spread_sig(const BlockSmem &b, uint32_t *wp, uint32_t &cw, int k, int sym) {
-  if (k == 0 && !causal_flag(b)) {
-    uint32_t *up = wp - b.gap;
-    up[-1] |= 0x100u << 9;
-    up[0] |= (0x80u << 9) | ((uint32_t)sym << 31);
-    up[1] |= 0x40u << 9;
-  } else if (k == 3) {
-    uint32_t *dn = wp + b.gap;
-    dn[-1] |= 0x04u;
-    dn[0] |= 0x02u | ((uint32_t)sym << 18);
-    dn[1] |= 0x01u;
+inline void build_t1_tables(T1Tables &T) {
+  static const uint16_t QE[47] = {0x5601, 0x3401, 0x1801, 0x0AC1, 0x0521, 0x0221, 0x5601, 0x5401, 0x4801, 0x3801,
+                                  0x3001, 0x2401, 0x1C01, 0x1601, 0x5601, 0x5401, 0x5101, 0x4801, 0x3801, 0x3401,
+                                  0x3001, 0x2801, 0x2401, 0x2201, 0x1C01, 0x1801, 0x1601, 0x1401, 0x1201, 0x1101,
+                                  0x0AC1, 0x09C1, 0x08A1, 0x0521, 0x0441, 0x02A1, 0x0221, 0x0141, 0x0111, 0x0085,
+                                  0x0049, 0x0025, 0x0015, 0x0009, 0x0005, 0x0001, 0x5601};
+  static const uint8_t NMPS[47] = {1,  2,  3,  4,  5,  38, 7,  8,  9,  10, 11, 12, 13, 29, 15, 16,
+                                   17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32,
+                                   33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 45, 46};
+  static const uint8_t NLPS[47] = {1,  6,  9,  12, 29, 33, 6,  14, 14, 14, 17, 18, 20, 21, 14, 14,
+                                   15, 16, 17, 18, 19, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29,
+                                   30, 31, 32, 33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43, 46};
+  std::memset(&T, 0, sizeof(T));
+  auto entry = [&](int s) {
+    uint2 e;
+    e.x = (uint32_t)QE[s >> 1] << 8;
+    e.y = ((uint32_t)(s & 1) << 31) | (uint32_t)(s * sizeof(T.mq[0]));
+    return e;
+  };
+  for (int s = 0; s < 94; ++s) {
+    const int idx = s >> 1, mps = s & 1;
+    const int sw = QE[idx] == 0x5601 && NLPS[idx] != 46;
+    T.mq[s][0] = entry(s);
+    T.mq[s][1] = entry(NMPS[idx] << 1 | mps);
+    T.mq[s][2] = entry(NLPS[idx] << 1 | (mps ^ sw));
   }
-  wp[-1] |= 0x20u << (3 * k);
-  wp[1] |= 0x08u << (3 * k);
-  cw |= ROW_SIG(k) | ((uint32_t)sym << (CHI_POS + 3 * k));
+  for (int band = 0; band < 3; ++band)
+    for (int nb = 0; nb < 512; ++nb) {
+      int h = ((nb >> 3) & 1) + ((nb >> 5) & 1);
+      int v = ((nb >> 1) & 1) + ((nb >> 7) & 1);
+      int d = (nb & 1) + ((nb >> 2) & 1) + ((nb >> 6) & 1) + ((nb >> 8) & 1);
+      int c;
+      if (band == 2) {  // HH
+        int hv = h + v;
+        if (d >= 3) c = 8;
+        else if (d == 2) c = hv >= 1 ? 7 : 6;
+        else if (d == 1) c = hv >= 2 ? 5 : (hv == 1 ? 4 : 3);
+        else c = hv >= 2 ? 2 : hv;
+      } else {
+        if (band == 1) std::swap(h, v);  // HL
+        if (h == 2) c = 8;
+        else if (h == 1) c = v >= 1 ? 7 : (d >= 1 ? 6 : 5);
+        else if (v == 2) c = 4;
+        else if (v == 1) c = 3;
+        else c = d >= 2 ? 2 : d;
+      }
+      T.zc[band][nb] = (uint8_t)((C_SIG + c) * SLOT);
+    }
+  for (int i = 0; i < 256; ++i) {
+    // bit 0 sigma up, 1 chi up, 2 sigma down, 3 chi down, 4 sigma left, 5 chi left,
+    // 6 sigma right, 7 chi right (T.800 Table D.3)
+    auto contrib = [&](int sb, int xb) { return ((i >> sb) & 1) ? (((i >> xb) & 1) ? -1 : 1) : 0; };
+    int H = contrib(4, 5) + contrib(6, 7);
+    int V = contrib(0, 1) + contrib(2, 3);
+    H = H < -1 ? -1 : (H > 1 ? 1 : H);
+    V = V < -1 ? -1 : (V > 1 ? 1 : V);
+    int x = 0;
+    if (H < 0 || (H == 0 && V < 0)) {
+      H = -H;
+      V = -V;
+      x = 1;
+    }
+    const int c = (H == 1) ? (V == 1 ? 4 : (V == 0 ? 3 : 2)) : (V == 1 ? 1 : 0);
+    static const int at[8] = {1, 16, 7, 22, 4, 19, 6, 21};  // their places in sign_index()
+    uint32_t w = 0;
+    for (int k = 0; k < 8; ++k) w |= (uint32_t)((i >> k) & 1) << at[k];
+    T.sc[sign_fold(w)] = (uint8_t)((C_SIGN + c) * SLOT | x);
+  }
 }
 
 enum { P_SIGPROP = 0, P_MAGREF = 1, P_CLEANUP = 2 };
 
-// one decision: a raw bit in a bypass segment, else an MQ symbol
-template <bool UNROLLED>
-__device__ __forceinline__ int decide(bool israw, Raw &raw, Mq &mq, uint2 *slot, const uint2 *tab) {
-  return israw ? raw_bit(raw) : mq_decode<!UNROLLED>(mq, slot, tab);
+// Rows with a significant sample in their 3 x 3 neighbourhood, the own bit included
+__device__ __forceinline__ uint32_t near_rows(uint32_t w) {
+  const uint32_t y = w | (w >> 1) | (w >> 2);
+  return (y | (y >> 3) | (y >> 6)) & ROWS;
 }
 
-// Sign of row k (raw bit, or MQ symbol in the sign context of its neighbours XOR the
-// context's prediction bit), then the sample becomes significant; returns its column update
-template <bool UNROLLED>
-__device__ __forceinline__ uint32_t significant(const BlockSmem &b, uint32_t *wp, uint32_t &cw, int k, bool israw,
-                                                Raw &raw, Mq &mq, const T1Tables &T) {
-  int flip = 0, slot = C_SIGN;
-  if (!israw) {
-    const int sv = T.sc[sign_index(cw, wp[-1], wp[1], k)];
-    slot += sv >> 1;
-    flip = sv & 1;
-  }
-  const int sg = decide<UNROLLED>(israw, raw, mq, b.cx + slot, T.mq) ^ flip;
-  spread_sig(b, wp, cw, k, sg);
-  return (1u << k) | ((uint32_t)sg << (4 + k));  // this row's column update
+// List positions of a chunk: the lanes' row sets x, columns in lane order, rows downwards;
+// returns the number of entries, `pos` the lane's first
+__device__ __forceinline__ int list_positions(uint32_t x, int lane, int &pos, uint4 &rows) {
+  rows.x = __ballot_sync(0xffffffffu, x & 1u);
+  rows.y = __ballot_sync(0xffffffffu, x & 8u);
+  rows.z = __ballot_sync(0xffffffffu, x & 0x40u);
+  rows.w = __ballot_sync(0xffffffffu, x & 0x200u);
+  const uint32_t lt = (1u << lane) - 1u;
+  pos = __popc(rows.x & lt) + __popc(rows.y & lt) + __popc(rows.z & lt) + __popc(rows.w & lt);
+  return __popc(rows.x) + __popc(rows.y) + __popc(rows.z) + __popc(rows.w);
 }
 
-// Rows of a stripe column that pass a pass's test, as a 4-bit mask (bit k = row k), with
-// v = word >> 3k holding row k's bits at row 0's positions:
-// (v & FORBID) == 0 && (v & NEED) == NEED && (ANY == 0 || (v & ANY) != 0)
-template <uint32_t FORBID, uint32_t NEED, uint32_t ANY>
-__device__ __forceinline__ uint32_t row_mask(uint32_t cw) {
-  uint32_t m = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t v = cw >> (3 * k);
-    const bool ok = !(v & FORBID) && (v & NEED) == NEED && (ANY == 0 || (v & ANY) != 0);
-    m |= (uint32_t)ok << k;
-  }
-  return m;
+// Significance propagation (bmi_block_decoder.cpp:10-215): samples not yet significant with a
+// significant neighbour.  Cleanup (:351-586): every sample not yet coded in this bit-plane; an
+// all-zero column is one run-length symbol (if it is 1, two uniform symbols give the row of
+// the first significant sample, whose sign follows directly).  A sample that becomes
+// significant changes the words around it, so the walk goes column by column from the words
+// themselves; the lanes only tell which columns of a chunk have work, and a column right of a
+// new significant sample joins them.
+// PASS and RAW (a bypass segment: raw bits instead of MQ symbols) are compile-time constants.
+// Predicated stores without a branch (a branch on which the lanes differ costs the warp tens
+// of cycles): a sample's first value, from the lane that owns its column (the same lane issues
+// the sample's refinements, so its updates stay in order), a refinement, and a list label
+__device__ __forceinline__ void put_sample(uint32_t *at, uint32_t v, uint32_t on) {
+#ifdef __CUDACC__
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(at), "r"(v), "r"(on)
+               : "memory");
+#else
+  if (on) *at = v;
+#endif
 }
-constexpr uint32_t V_SIG = 0x10u, V_CHI = 1u << CHI_POS, V_MU = 1u << MU_POS, V_PI = 1u << PI_POS;
-
-// Two forms of each pass's column code, with identical decisions:
-//   UNROLLED = false (throughput): the rows to visit are a 4-bit mask walked with ffs, and
-//     each decision is inlined once, so the kernel stays small for the instruction cache
-//     when many warps are resident and sit in different passes;
-//   UNROLLED = true (latency): the four rows are unrolled with constant masks, trading
-//     code size for a shorter dependency chain per symbol, for batches too small to fill
-//     the GPU, whose time is the serial time of their longest blocks.
-
-// significance propagation of one stripe column (bmi_block_decoder.cpp:10-215): rows
-// not yet significant with a significant neighbour; a row that becomes significant can
-// make the rows below it eligible
-template <bool UNROLLED>
-__device__ __forceinline__ uint32_t sigprop_column(const BlockSmem &b, uint32_t *wp, uint32_t &cw, uint32_t todo,
-                                                   bool israw, const uint8_t *zc, Raw &raw, Mq &mq,
-                                                   const T1Tables &T) {
-  uint32_t upd = 0;
-  if constexpr (UNROLLED) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t v = cw >> (3 * k);
-      if (!(v & NBR_ROW0) || (v & (V_SIG | V_CHI))) continue;
-      const int d = decide<UNROLLED>(israw, raw, mq, b.cx + C_SIG + zc[v & NBR_ROW0], T.mq);
-      cw |= ROW_PI(k);
-      if (d) upd |= significant<UNROLLED>(b, wp, cw, k, israw, raw, mq, T);
-    }
-  } else {
-    while (todo) {
-      const int k = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int d = decide<UNROLLED>(israw, raw, mq, b.cx + C_SIG + zc[(cw >> (3 * k)) & NBR_ROW0], T.mq);
-      cw |= ROW_PI(k);
-      if (d) {
-        upd |= significant<UNROLLED>(b, wp, cw, k, israw, raw, mq, T);
-        todo = row_mask<V_SIG | V_CHI, 0u, NBR_ROW0>(cw) & (0xEu << k);
-      }
-    }
-  }
-  return upd;
+__device__ __forceinline__ void flip_sample(uint32_t *at, uint32_t v, uint32_t on) {
+#ifdef __CUDACC__
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.global.xor.b32 [%0], %1;\n\t}" ::"l"(at), "r"(v),
+               "r"(on)
+               : "memory");
+#else
+  if (on) *at ^= v;
+#endif
+}
+__device__ __forceinline__ void put_label(uint8_t *at, uint32_t v, uint32_t on) {
+#ifdef __CUDACC__
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p st.shared.u8 [%0], %1;\n\t}" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(at)),
+               "r"(v), "r"(on)
+               : "memory");
+#else
+  if (on) *at = (uint8_t)v;
+#endif
 }
 
-// magnitude refinement of one stripe column (bmi_block_decoder.cpp:217-349): rows
-// significant before this bit-plane
-template <bool UNROLLED>
-__device__ __forceinline__ uint32_t magref_column(const BlockSmem &b, uint32_t cw, uint32_t rows, uint8_t *rf,
-                                                  bool israw, Raw &raw, Mq &mq, const T1Tables &T) {
-  const uint32_t refined = *rf;
-  uint32_t bits = 0;
-  if (israw) {
-    // bypass: the column's refinement bits are consecutive raw bits, taken together
-    const int n = __popc(rows);
-    uint32_t x = 0;
-    if (raw.ct >= n) {
-      x = (raw.c >> (raw.ct - n)) & ((1u << n) - 1u);
-      raw.ct -= n;
-    } else {
-      for (int i = 0; i < n; ++i) x = (x << 1) | (uint32_t)raw_bit(raw);
-    }
-    if (rows) *rf = (uint8_t)(refined | rows);
-    return rows | ((uint32_t)T.rawmr[rows][x] << 4);
-  }
-#pragma unroll
-  for (int i = 0; i < (UNROLLED ? 4 : 1); ++i) {
-    uint32_t todo = UNROLLED ? (rows & (1u << i)) : rows;
-    while (todo) {
-      const int k = UNROLLED ? i : __ffs(todo) - 1;
-      todo &= todo - 1;
-      // first refinement of this sample <=> (|v| >> p) < 4 in the reference
-      const int ctx = C_MAG + (((refined >> k) & 1) ? 2 : (((cw >> (3 * k)) & NBR_ROW0) ? 1 : 0));
-      bits |= (uint32_t)decide<UNROLLED>(israw, raw, mq, b.cx + ctx, T.mq) << (4 + k);
-    }
-  }
-  if (rows) *rf = (uint8_t)(refined | rows);
-  return rows | bits;  // column update: rows refined and their decoded bits
+template <int PASS>
+__device__ __forceinline__ uint32_t pass_rows(uint32_t word) {
+  if (PASS == P_SIGPROP) return near_rows(word) & ~((word >> SIG_POS) | (word >> CHI_POS));
+  return ~((word >> SIG_POS) | (word >> CHI_POS) | (word >> PI_POS)) & ROWS;
 }
 
-// cleanup of one stripe column (bmi_block_decoder.cpp:351-586): an all-zero column is
-// coded in run mode (one run-length symbol; if it is 1, two uniform symbols give the row
-// of the first significant sample, whose sign follows directly); then every row not yet
-// coded in this bit-plane
-template <bool UNROLLED>
-__device__ __forceinline__ uint32_t cleanup_column(const BlockSmem &b, uint32_t *wp, uint32_t &cw, uint32_t todo,
-                                                   const uint8_t *zc, Raw &raw, Mq &mq, const T1Tables &T) {
-  int forced = -1;
-  if (cw == 0) {
-    // run-length symbol, then the two uniform symbols (the reference's fixed-Qe
-    // MQ_DECODE_START is an ordinary decision on a context pinned at state 46)
-    int r = 0;
-#pragma unroll 1
-    for (int i = 0; i < 3; ++i) {
-      const int d = mq_decode<!UNROLLED>(mq, b.cx + (i == 0 ? C_RUN : C_UNI), T.mq);
-      if (i == 0 && !d) return 0;  // the whole column stays insignificant
-      r = (r << 1) | d;
-    }
-    forced = r & 3;
-    todo = (0xFu << forced) & 0xFu;
-  }
-  uint32_t upd = 0;
-#pragma unroll
-  for (int i = 0; i < (UNROLLED ? 4 : 1); ++i) {
-    uint32_t rows = UNROLLED ? (todo & (1u << i)) : todo;
-    while (rows) {
-      const int k = UNROLLED ? i : __ffs(rows) - 1;
-      rows &= rows - 1;
-      if (k != forced && !mq_decode<!UNROLLED>(mq, b.cx + C_SIG + zc[(cw >> (3 * k)) & NBR_ROW0], T.mq)) continue;
-      upd |= significant<UNROLLED>(b, wp, cw, k, false, raw, mq, T);
-    }
-  }
-  return upd;
-}
-
-// One coding pass over the block.  Columns are visited in 32-column chunks: a ballot
-// selects the columns with work (non-zero word for significance propagation, a refinable
-// sample for refinement, every column for cleanup); a sample that becomes significant makes
-// the next column non-zero, so that column joins the set.  In cleanup, a run of all-zero
-// columns whose run-length symbols would all decode as MPS without renormalisation
-// (C >= k*Qe and A - k*Qe >= 0x8000, scaled) is consumed in one step: A -= k*Qe, C -= k*Qe.
-// Each pass inlines its decision sites once, without unrolling over the four rows, so the
-// kernel stays small enough for the instruction cache when many warps are resident.
-// PASS (P_SIGPROP / P_MAGREF / P_CLEANUP) and RAW (a bypass segment: raw bits instead of MQ
-// symbols) are compile-time constants, so each instantiation carries only its own pass's
-// column code and no decision tests either flag at run time.
-template <bool UNROLLED, int PASS, bool RAW>
-__device__ __forceinline__ void run_pass(const BlockSmem &b, int stripes, int p, const uint8_t *zc, Mq &mq, Raw &raw,
-                                         const T1Tables &T, int lane) {
-  constexpr int pass = PASS;
-  constexpr bool israw = RAW;
-  for (int s = 0; s < stripes; ++s) {
-    uint32_t *row = cword(b, s, 0);
-    uint8_t *rrow = b.rf + s * b.gap;
+template <bool LATENCY, int PASS, bool RAW>
+__device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq, Raw &raw) {
+  const int lane = b.lane;
+  for (int s = 0; s < b.stripes; ++s) {
+    uint32_t *row = b.cw + s * b.gap;
+    uint32_t *out = b.out + (size_t)(4 * s) * b.stride;
     for (int c0 = 0; c0 < b.w; c0 += 32) {
       __syncwarp();
-      // lane-parallel view of the chunk: each lane's word and the rows its pass would
-      // visit; only columns with work join the serial loop (a column reached from the left
-      // by a new significant sample joins it then).  The unrolled form also hands the
-      // lanes' words and masks to the serial loop: a column's word changes only when its
-      // left neighbour gains a significant sample (`dirty`), so only those are reloaded.
-      // The compact form keeps fewer values live across the serial loop (registers bound
-      // its occupancy) and reloads each word.
-      constexpr bool LP = UNROLLED;
-      const int c = c0 + lane;
-      const bool valid = c < b.w;
-      const uint32_t word = valid ? row[c] : 0u;
-      uint32_t mask;
-      bool work;
-      if (pass == P_SIGPROP) {
-        mask = row_mask<V_SIG | V_CHI, 0u, NBR_ROW0>(word);
-        work = mask != 0;
-      } else if (pass == P_MAGREF) {
-        mask = row_mask<0u, V_SIG | V_MU, 0u>(word);
-        work = mask != 0;
-      } else {
-        mask = row_mask<V_SIG | V_CHI | V_PI, 0u, 0u>(word);
-        work = word == 0 || mask != 0;  // run mode, or rows not yet coded in this bit-plane
-      }
-      uint32_t live = __ballot_sync(0xffffffffu, valid && work);
-      uint32_t zero = __ballot_sync(0xffffffffu, valid && word == 0);
-      uint32_t dirty = 0;
-      uint32_t my_upd = 0;  // this lane's column update, flushed at the end of the chunk
-      // compact form: the lanes' cleanup / refinement masks go through shared memory (they
-      // depend on a column's own rows only, so they hold while the chunk is decoded; a
-      // register copy would raise the register count above the occupancy budget)
-      uint8_t *lane_masks = reinterpret_cast<uint8_t *>(b.cx + N_CTX);
-      if (!LP && pass != P_SIGPROP) {
-        lane_masks[lane] = (uint8_t)mask;
-        __syncwarp();
-      }
+      const bool valid = c0 + lane < b.w;
+      const uint32_t word = valid ? row[c0 + lane] : 0u;
+      uint32_t *mine = out + c0 + lane;
+      uint32_t live = __ballot_sync(0xffffffffu, valid && pass_rows<PASS>(word));
+      uint32_t zero = PASS == P_CLEANUP ? __ballot_sync(0xffffffffu, valid && word == 0) : 0u;
+      const uint32_t inside = b.w - c0 >= 32 ? 0xffffffffu : (1u << (b.w - c0)) - 1u;
       while (live) {
         const int bit = __ffs(live) - 1;
-        if (pass == P_CLEANUP && ((zero >> bit) & 1)) {
-          const uint2 e = b.cx[C_RUN];
-          const int32_t q = (int32_t)e.x;
-          const int32_t m = min(mq.A - 0x800000, mq.C);
-          if (!((e.y >> 16) & 1) && m >= q) {
-            int n = __clz(__brev(~(zero >> bit)));  // zero columns from `bit` on, in this chunk
-            if (n * q > m) n = m / q;
+        uint32_t *wp = row + c0 + bit;
+        uint32_t W = *wp, x, k3 = 0;
+        bool forced = false;
+        if (PASS == P_CLEANUP && ((zero >> bit) & 1)) {
+          uint2 e = *reinterpret_cast<const uint2 *>(b.cx + RUN_OFF);
+          const int32_t q = (int32_t)e.x, room = min(mq.A - A_MIN, mq.C);
+          if (!(e.y >> 31) && room >= q) {
+            // zero columns from here on: as many as need no renormalisation
+            int n = __clz(__brev(~(zero >> bit)));
+            if (n * q > room) n = room / q;
             mq.A -= n * q;
             mq.C -= n * q;
-            const uint32_t span = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
-            live &= ~(span << bit);
+            live &= ~((n >= 32 ? 0xffffffffu : (1u << n) - 1u) << bit);
             continue;
           }
-        }
-        live &= live - 1;
-        const int col = c0 + bit;
-        uint32_t *wp = row + col;
-        uint32_t cw, lane_word = 0, lane_mask = 0;
-        bool dty = true;
-        if (LP) {
-          lane_word = __shfl_sync(0xffffffffu, word, bit);
-          lane_mask = __shfl_sync(0xffffffffu, mask, bit);
-          dty = (dirty >> bit) & 1;
-          cw = dty ? *wp : lane_word;
+          live &= live - 1;
+          mq_ready(mq);
+          if (!mq_symbol<LATENCY>(mq, b.cx + RUN_OFF, e, b.mq)) continue;
+          k3 = mq_decode<LATENCY>(mq, b.cx, UNI_OFF, b.mq) * 6;
+          k3 += mq_decode<LATENCY>(mq, b.cx, UNI_OFF, b.mq) * 3;
+          x = ROWS & (0xFFFFFFF8u << k3);
+          forced = true;
         } else {
-          cw = *wp;
+          live &= live - 1;
+          x = pass_rows<PASS>(W);
+          if (PASS == P_SIGPROP) W |= x << PI_POS;
         }
-        if (pass == P_MAGREF) {
-          const uint32_t rows = LP ? lane_mask : lane_masks[bit];
-          const uint32_t upd = magref_column<UNROLLED>(b, cw, rows, rrow + col, israw, raw, mq, T);
-          if constexpr (UNROLLED) my_upd = lane == bit ? upd : my_upd;
-          else b.sp.apply<true>(4 * s, col, upd, p);
-          continue;
+        uint32_t hit = 0;
+        while (forced || x) {
+          if (!forced) {
+            k3 = __ffs(x) - 1;
+            x &= x - 1;
+            uint32_t d;
+            if (RAW) {
+              d = raw_bit(raw);
+            } else {
+              const uint32_t off = b.zc[(W >> k3) & 0x1EF];
+              uint2 e = *reinterpret_cast<const uint2 *>(b.cx + off);
+              mq_ready(mq);
+              d = mq_symbol<LATENCY>(mq, b.cx + off, e, b.mq);
+            }
+            if (!d) continue;
+          }
+          forced = false;
+          // row k3 / 3 becomes significant: sign, neighbours, first value
+          uint32_t sign;
+          if (RAW) {
+            sign = raw_bit(raw);
+          } else {
+            const uint32_t sv = b.sc[sign_index(W, wp[-1], wp[1], k3)], off = sv & 0xF8;
+            uint2 e = *reinterpret_cast<const uint2 *>(b.cx + off);
+            mq_level(mq);
+            sign = mq_symbol<LATENCY>(mq, b.cx + off, e, b.mq) ^ (sv & 1);
+          }
+          hit = 0xffffffffu;
+          W |= ((1u << SIG_POS) | (sign << CHI_POS)) << k3;
+          __syncwarp();
+          spread(b, wp, k3, sign);
+          __syncwarp();
+          // (the latency form keeps its lane's column address, the throughput form the registers)
+          put_sample((LATENCY ? mine : out + c0 + bit) + (k3 * 11 >> 5) * b.stride, (sign << 31) + (3u << p >> 1),
+                     lane == bit);
+          if (PASS == P_SIGPROP) {
+            x = pass_rows<PASS>(W) & (0xFFFFFFF8u << k3);
+            W |= x << PI_POS;
+          }
         }
-        uint32_t upd;
-        if (pass == P_SIGPROP) {
-          const uint32_t todo = dty ? row_mask<V_SIG | V_CHI, 0u, NBR_ROW0>(cw) : lane_mask;
-          upd = sigprop_column<UNROLLED>(b, wp, cw, todo, israw, zc, raw, mq, T);
-        } else {
-          // own-row bits do not change from the left, so the lane's mask holds; a column
-          // that was all-zero may have been reached from the left and is not any more
-          const uint32_t todo = LP ? ((dty && lane_word == 0) ? row_mask<V_SIG | V_CHI | V_PI, 0u, 0u>(cw) : lane_mask)
-                                   : lane_masks[bit];
-          upd = cleanup_column<UNROLLED>(b, wp, cw, todo, zc, raw, mq, T);
-        }
-        *wp = cw;
-        const bool newsig = (upd & 0xF) != 0;
-        if constexpr (UNROLLED) my_upd = lane == bit ? upd : my_upd;
-        else if (newsig) b.sp.apply<false>(4 * s, col, upd, p);
-        if (newsig && bit < 31) {
-          if (pass == P_SIGPROP) live |= 1u << (bit + 1);
-          zero &= ~(1u << (bit + 1));
-          if (LP) dirty |= 1u << (bit + 1);
-        }
+        *wp = W;
+        const uint32_t right = (2u << bit) & inside & hit;
+        if (PASS == P_SIGPROP) live |= right;
+        else zero &= ~right;
       }
-      if constexpr (UNROLLED) b.sp.flush<pass == P_MAGREF>(4 * s, c, my_upd, p);
-      if (pass == P_CLEANUP) {
+      if (PASS == P_CLEANUP) {
         // end of the bit-plane for this chunk's columns: mu |= sigma, pi cleared
-        // (bmi_block_decoder.cpp:571-573); no later decision of this pass reads a column's
-        // own mu / pi bits
+        // (bmi_block_decoder.cpp:571-573); no later symbol of this pass reads a column's own
+        // mu / pi bits
         __syncwarp();
         if (valid) {
-          uint32_t w = row[c];
-          w |= (w << (MU_POS - 4)) & MU_ALL;
-          row[c] = w & ~PI_ALL;
+          const uint32_t w = row[c0 + lane];
+          row[c0 + lane] = (w | ((w << (MU_POS - SIG_POS)) & MU_ALL)) & ~PI_ALL;
         }
       }
     }
@@ -609,12 +564,153 @@ __device__ __forceinline__ void run_pass(const BlockSmem &b, int stripes, int p,
   __syncwarp();
 }
 
-__device__ __forceinline__ void init_states(uint2 *cx, const uint2 *tab) {
+// The refinement symbols of a chunk: n labels in scan order, decoded bits to b.bits.  The
+// latency form takes four at a time: their slots are loaded together and entries changed
+// within the four passed on in registers, so no symbol waits for a store and a load.
+template <bool LATENCY>
+__device__ __forceinline__ void refine(const Block &b, const uint8_t *list, int n, Mq &mq) {
+  uint8_t *cx = b.cx + C_MAG * SLOT;
+  uint32_t bits = 0;
+  int i = 0;
+  if (LATENCY) {
+    const uint32_t *four = reinterpret_cast<const uint32_t *>(list);
+    uint32_t next = four[0];
+    constexpr uint32_t ALL2 = 2 * SLOT * 0x01010101u;
+    while (i + 4 <= n) {
+      if (next == ALL2) {
+        // every sample refined before: one context, its entry in registers
+        uint2 e = *reinterpret_cast<const uint2 *>(cx + 2 * SLOT);
+        bool more;
+        do {
+          if (mq.T < T_MIN && !mq_refill(mq)) break;
+          next = four[(i >> 2) + 1];
+          uint32_t d = mq_symbol<true, false>(mq, cx, e, b.mq);
+          d |= mq_symbol<true, false>(mq, cx, e, b.mq) << 1;
+          if (mq.T < T_MIN && !mq_refill(mq)) {
+            *reinterpret_cast<uint2 *>(cx + 2 * SLOT) = e;  // a carry waits
+            bits |= d << (i & 31);
+            i += 2;
+            goto singles;
+          }
+          d |= mq_symbol<true, false>(mq, cx, e, b.mq) << 2;
+          d |= mq_symbol<true, false>(mq, cx, e, b.mq) << 3;
+          bits |= d << (i & 31);
+          i += 4;
+          if (!(i & 31)) {
+            b.bits[(i >> 5) - 1] = bits;
+            bits = 0;
+          }
+          more = next == ALL2 && i + 4 <= n;
+        } while (more);
+        *reinterpret_cast<uint2 *>(cx + 2 * SLOT) = e;
+        if (mq.T < T_MIN && !mq_refill(mq)) break;
+        continue;
+      }
+      const uint32_t o = next;
+      const uint32_t o0 = o & 0xFF, o1 = (o >> 8) & 0xFF, o2 = (o >> 16) & 0xFF, o3 = o >> 24;
+      uint2 e0 = *reinterpret_cast<const uint2 *>(cx + o0), e1 = *reinterpret_cast<const uint2 *>(cx + o1),
+            e2 = *reinterpret_cast<const uint2 *>(cx + o2), e3 = *reinterpret_cast<const uint2 *>(cx + o3);
+      next = four[(i >> 2) + 1];
+      if (mq.T < T_MIN && !mq_refill(mq)) break;
+      uint32_t d = mq_symbol<true>(mq, cx + o0, e0, b.mq);
+      if (o1 == o0) e1 = e0;
+      d |= mq_symbol<true>(mq, cx + o1, e1, b.mq) << 1;
+      bits |= d << (i & 31);
+      i += 2;
+      if (mq.T < T_MIN && !mq_refill(mq)) break;
+      if (o2 == o0) e2 = e0;
+      if (o2 == o1) e2 = e1;
+      d = mq_symbol<true>(mq, cx + o2, e2, b.mq);
+      if (o3 == o0) e3 = e0;
+      if (o3 == o1) e3 = e1;
+      if (o3 == o2) e3 = e2;
+      d |= mq_symbol<true>(mq, cx + o3, e3, b.mq) << 1;
+      bits |= d << (i & 31);
+      i += 2;
+      if (!(i & 31)) {
+        b.bits[(i >> 5) - 1] = bits;
+        bits = 0;
+      }
+    }
+  }
+singles:
+  // one at a time: the throughput form, a chunk's last three, and while a carry waits
+  for (; i < n; ++i) {
+    bits |= mq_decode<LATENCY>(mq, cx, list[i], b.mq) << (i & 31);
+    if ((i & 31) == 31) {
+      b.bits[i >> 5] = bits;
+      bits = 0;
+    }
+  }
+  if (n & 31) b.bits[n >> 5] = bits;
+}
+
+// Magnitude refinement (bmi_block_decoder.cpp:217-349): samples significant before this
+// bit-plane.  The reference's "first refinement" test (|v| >> p) < 4 is true exactly on a
+// sample's first refinement: a bit per sample in `rf`.
+template <bool LATENCY, bool RAW>
+__device__ __forceinline__ void refinement_pass(const Block &b, int p, Mq &mq, Raw &raw) {
+  const int lane = b.lane;
+  uint8_t *list = b.list;
+  const int chunks = (b.w + 31) >> 5;
+  for (int s = 0; s < b.stripes; ++s) {
+    for (int h = 0; h < chunks; ++h) {
+      const int c = h * 32 + lane;
+      const uint32_t word = c < b.w ? b.cw[s * b.gap + c] : 0u;
+      const uint32_t x = (word >> SIG_POS) & (word >> MU_POS) & ROWS;
+      if (!__any_sync(0xffffffffu, x)) continue;
+      int pos;
+      uint4 rows;
+      const int n = list_positions(x, lane, pos, rows);
+      uint4 rf = b.rf[s * chunks + h];
+      int at = pos;
+      if (!RAW) {
+        // label: 2 once refined, else 1 with a significant neighbour
+        const uint32_t y = word | (word >> 1) | (word >> 2);
+        const uint32_t near = y | (y >> 6) | (word >> 3) | (word >> 5);
+        put_label(list + at, (rf.x >> lane) & 1 ? 2 * SLOT : (near & 1u) * SLOT, x & 1u);
+        at += x & 1u;
+        put_label(list + at, (rf.y >> lane) & 1 ? 2 * SLOT : ((near >> 3) & 1u) * SLOT, x & 8u);
+        at += (x >> 3) & 1u;
+        put_label(list + at, (rf.z >> lane) & 1 ? 2 * SLOT : ((near >> 6) & 1u) * SLOT, x & 0x40u);
+        at += (x >> 6) & 1u;
+        put_label(list + at, (rf.w >> lane) & 1 ? 2 * SLOT : ((near >> 9) & 1u) * SLOT, x & 0x200u);
+      }
+      __syncwarp();
+      rf.x |= rows.x;
+      rf.y |= rows.y;
+      rf.z |= rows.z;
+      rf.w |= rows.w;
+      if (lane == 0) b.rf[s * chunks + h] = rf;
+      if (RAW) {
+        for (int i = 0; i < n; i += 32) b.bits[i >> 5] = raw_bits(raw, min(32, n - i));
+      } else {
+        refine<LATENCY>(b, list, n, mq);
+      }
+      __syncwarp();
+      // each lane's samples: bit p as decoded, the next midpoint bit
+      unsigned int *col = b.out + (size_t)(4 * s) * b.stride + c;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t on = x & (1u << (3 * k));
+        const uint32_t d = (b.bits[(pos >> 5) & 3] >> (pos & 31)) & 1;  // unused (and in bounds) when off
+        pos += on ? 1 : 0;
+        flip_sample(col + (size_t)k * b.stride, ((1u - d) << p) | ((1u << p) >> 1), on);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// (every lane writes the same)
+__device__ __forceinline__ void init_states(uint8_t *cx, const uint8_t *tab) {
   // bmi_mq_decoder.cpp:65-79: (state 0, MPS 0) except sig ctx 0 -> state 4, run -> state 3
-  for (int i = 0; i < N_CTX; ++i) cx[i] = tab[0];
-  cx[C_SIG] = tab[4 << 1];
-  cx[C_RUN] = tab[3 << 1];
-  cx[C_UNI] = tab[46 << 1];
+  const uint2(*t)[3] = reinterpret_cast<const uint2(*)[3]>(tab);
+  uint2 *slot = reinterpret_cast<uint2 *>(cx);
+  for (int i = 0; i < N_CTX; ++i) slot[i] = t[0][0];
+  slot[C_SIG] = t[4 << 1][0];
+  slot[C_RUN] = t[3 << 1][0];
+  slot[C_UNI] = t[46 << 1][0];
 }
 
 __device__ __forceinline__ bool seg_starts(int flags, int j) {
@@ -640,45 +736,43 @@ __device__ __forceinline__ void block_planes(const j2k_cblk &cb, int &bit_plane,
   if (bit_plane == 0) bit_plane = 1;
 }
 
-// Decode one code-block with the whole warp.  Returns a status (0 ok).
-template <bool UNROLLED>
-__device__ __forceinline__ int decode_block(const j2k_cblk &cb, const uint8_t *__restrict__ bytes, const uint32_t *__restrict__ seglens,
-                            const BlockSmem &b, const T1Tables &T, int lane, int bit_plane, int num_passes) {
-  const int w = cb.w, h = cb.h;
-  const int stripes = (h + 3) >> 2;
-  // clear the context words and refinement bits (the samples need no clearing: see
-  // Samples); mark OOB columns and a partial last stripe
+// Decode one code-block with the whole warp: raw sign-magnitude samples in b.out, the
+// significance of every sample in the context words.  Returns a status (0 ok).
+template <bool LATENCY>
+__device__ __forceinline__ int decode_block(const j2k_cblk &cb, const uint8_t *__restrict__ bytes,
+                                            const uint32_t *__restrict__ seglens, Block &b, int bit_plane,
+                                            int num_passes) {
+  const int w = cb.w, h = cb.h, lane = b.lane;
+  const int stripes = b.stripes;
+  // clear the context words and refinement bits (the samples need no clearing: the final
+  // rewrite gives 0 to those that never became significant); mark columns and rows outside
+  // the block
+  uint32_t *first = b.cw - b.gap - 1;
   const int nwords = (stripes + 2) * b.gap + 2;
-  for (int i = lane; i < nwords; i += 32) b.cw[i] = 0;
-  for (int i = lane; i < stripes * b.gap; i += 32) b.rf[i] = 0;
+  for (int i = lane; i < nwords; i += 32) first[i] = 0;
+  for (int i = lane; i < stripes * ((w + 31) >> 5); i += 32) b.rf[i] = make_uint4(0, 0, 0, 0);
   __syncwarp();
-  const uint32_t oob = CHI_ALL;
   for (int s = lane; s < stripes; s += 32) {
-    uint32_t *r = cword(b, s, w);
-    r[0] = oob;
-    r[1] = oob;
-    r[2] = oob;
+    uint32_t *r = b.cw + s * b.gap + w;
+    r[0] = CHI_ALL;
+    r[1] = CHI_ALL;
+    r[2] = CHI_ALL;
   }
   if (h & 3) {
-    uint32_t m = (h & 3) == 1 ? (ROW_CHI(1) | ROW_CHI(2) | ROW_CHI(3))
-                              : ((h & 3) == 2 ? (ROW_CHI(2) | ROW_CHI(3)) : ROW_CHI(3));
-    for (int c = lane; c < w; c += 32) *cword(b, stripes - 1, c) = m;
+    const uint32_t m = CHI_ALL & (0xFFFFFFFFu << (CHI_POS + 3 * (h & 3)));
+    for (int c = lane; c < w; c += 32) b.cw[(stripes - 1) * b.gap + c] = m;
   }
-  if (lane == 0) {
-    init_states(b.cx, T.mq);
-    // stripe 0's refined-rows row has three unused bytes past the last column
-    causal_flag(b) = (cb.flags & J2K_CB_CAUSAL) ? 1 : 0;
-  }
+  init_states(b.cx, b.mq);
+  spread_init(b, (cb.flags & J2K_CB_CAUSAL) != 0);
   __syncwarp();
   if (num_passes > 0 && 30 - (int)cb.missing <= 0) return 1;
 
   const int multi = (cb.flags & (J2K_CB_BYPASS | J2K_CB_TERMALL)) != 0;
-  const uint8_t *zc = T.zc[cb.band == 3 ? 2 : (cb.band == 1 ? 1 : 0)];
   const uint8_t *data = bytes + cb.data_off;
   Mq mq;
   Raw raw;
-  mq.A = mq.C = mq.t = mq.T = 0;
-  mq.ap = mq.aend = mq.cur = mq.nxt = 0;
+  mq.A = mq.C = mq.T = 0;
+  mq.l0 = mq.l1 = mq.last = mq.ap = mq.aend = mq.cur = mq.nxt = 0;
   mq.w = reinterpret_cast<const uint32_t *>(bytes);
   raw_init(raw, data, 0);
   uint32_t seg_pos = 0;
@@ -715,16 +809,20 @@ __device__ __forceinline__ int decode_block(const j2k_cblk &cb, const uint8_t *_
       else mq_init(mq, data + seg_pos, len);
       seg_pos += len;
     }
-    if (type == P_CLEANUP) run_pass<UNROLLED, P_CLEANUP, false>(b, stripes, bit_plane, zc, mq, raw, T, lane);
-    else if (type == P_SIGPROP && israw) run_pass<UNROLLED, P_SIGPROP, true>(b, stripes, bit_plane, zc, mq, raw, T, lane);
-    else if (type == P_SIGPROP) run_pass<UNROLLED, P_SIGPROP, false>(b, stripes, bit_plane, zc, mq, raw, T, lane);
-    else if (israw) run_pass<UNROLLED, P_MAGREF, true>(b, stripes, bit_plane, zc, mq, raw, T, lane);
-    else run_pass<UNROLLED, P_MAGREF, false>(b, stripes, bit_plane, zc, mq, raw, T, lane);
-    if (type == 2 && (cb.flags & J2K_CB_SEGSYM))
-      for (int i = 0; i < 4; ++i) mq_uniform(mq);
+    if (type == P_CLEANUP) significance_pass<LATENCY, P_CLEANUP, false>(b, bit_plane, mq, raw);
+    else if (type == P_SIGPROP && israw) significance_pass<LATENCY, P_SIGPROP, true>(b, bit_plane, mq, raw);
+    else if (type == P_SIGPROP) significance_pass<LATENCY, P_SIGPROP, false>(b, bit_plane, mq, raw);
+    else if (israw) refinement_pass<LATENCY, true>(b, bit_plane, mq, raw);
+    else refinement_pass<LATENCY, false>(b, bit_plane, mq, raw);
+    if (type == 2 && (cb.flags & J2K_CB_SEGSYM)) {
+      // four uniform symbols (the reference's fixed-Qe MQ_DECODE_START, bmi_mq_decoder.h:131-169,
+      // is an ordinary symbol of a slot pinned at state 46)
+#pragma unroll 1
+      for (int i = 0; i < 4; ++i) mq_decode<LATENCY>(mq, b.cx, UNI_OFF, b.mq);
+    }
     if (cb.flags & J2K_CB_RESET) {
       __syncwarp();
-      if (lane == 0) init_states(b.cx, T.mq);
+      init_states(b.cx, b.mq);
       __syncwarp();
     }
   }
