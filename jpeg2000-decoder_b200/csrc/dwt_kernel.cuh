@@ -3,12 +3,20 @@
  * stage for sm_100a.
  *
  * One CTA reconstructs a 64x64 output tile of one resolution level of one
- * tile-component: it stages the 72x72 interleaved input window (the four quadrants of the
+ * tile-component: it stages the 72x72 interleaved window (the four quadrants of the
  * Mallat layout plus a 4-sample whole-sample-symmetric halo) in shared memory with
- * coalesced asynchronous copies, lifts each window row and then each output column in
- * registers (one thread streams one line), and writes
- * the 64x64 result with coalesced stores.  Every level is one read and one write of the
- * level's samples; all tile-components of a batch at a given level share one launch.
+ * coalesced asynchronous copies, lifts the window's rows and then its columns, a thread
+ * lifting eight outputs at a time in registers, and stores the 64x64 result from the column
+ * pass.  Every level is one read and one write of the level's samples; all tile-components
+ * of a batch at a given level share one launch.
+ * The kernels are bound by instruction issue (74 % of the slots in the 4096x2160 level, DRAM
+ * 1.0 TB/s) and, in small levels, by the latency of one tile, so the work is cut into short
+ * independent chains and the staging walks lines with pointers.  Measured on B200 against a
+ * thread per 72-sample line streamed through shared memory: a 4096x2160 9/7 plane of five
+ * levels 75.4 -> 45.7 us, a 1000x777 5/3 tile 43.8 -> 21.8 us (one cooperative launch with
+ * 32x32 tiles in the small levels; five launches of these kernels 61.6 and 32.8 us), the
+ * DWT + MCT stage of 32 1080p frames 0.955 -> 0.81 ms.  Five resident CTAs at 48 registers
+ * instead of four at 64 took 51.2 us (spills).
  *
  * Arithmetic follows the reference exactly so that results are bit-identical:
  *   9/7: each lifting update is D = S - c * (L + R) with three separately rounded float
@@ -23,15 +31,18 @@
  * reference's per-step mirroring at the region edges.
  */
 #pragma once
+#include <cooperative_groups.h>
+
 #include <cstdint>
 #include <type_traits>
+
+#include "plan.h"
 
 namespace j2k_dev {
 
 constexpr int DWT_T = 64;          // output tile edge
 constexpr int DWT_H = 4;           // halo
-constexpr int DWT_N = DWT_T + 2 * DWT_H;  // 72
-constexpr int DWT_PITCH = DWT_N + 1;      // odd pitch: conflict-free column access
+constexpr int DWT_PITCH = DWT_T + 2 * DWT_H + 1;  // of a 64x64 tile's window
 
 struct DwtLevel {
   uint64_t base;     // element offset of the tile-component region (same in every buffer)
@@ -75,12 +86,14 @@ struct OutTask {
   uint16_t tx, ty;
 };
 
+// Source position of window position p on a line of n samples: whole-sample symmetric
+// extension, which keeps the parity.  Positions more than four past the end feed no output:
+// they are brought back to one that exists.
 __device__ __forceinline__ int mirror(int p, int n) {
   if (n == 1) return 0;
-  const int period = 2 * (n - 1);
-  p %= period;
-  if (p < 0) p += period;
-  return p >= n ? period - p : p;
+  if (p > n + 3) p = n + 3 - ((n + 3 - p) & 1);
+  while (p < 0 || p >= n) p = p < 0 ? -p : 2 * (n - 1) - p;
+  return p;
 }
 
 __device__ __forceinline__ float lift97(float s, float c, float l, float r) {
@@ -98,56 +111,43 @@ struct DwtTypes<false> {
   typedef float T;
 };
 
-constexpr int DWT_THREADS = 128;    // threads per CTA of the level kernels
+constexpr int DWT_THREADS = 256;    // threads per CTA of the level kernels
 constexpr int FUSED_THREADS = 256;  // threads per CTA of the fused last-level + output kernel
 
-// Lifting of one window line (72 samples, element stride `st`), streamed by one thread
-// through registers: iteration m reads the pair (x[2m], x[2m+1]) and retires the samples
-// whose every lifting step is complete, in place behind the read position.  The values are
-// those of the step-by-step scheme that updates evens 2..70 and odds 1..69 in each step
-// (x[0] and x[71] keep their input values), which the 4-sample halo makes exact for the 64
-// centre positions; positions above 67 are not all written.
+// Inverse lifting of eight outputs of a line from the fifteen samples around them, in
+// registers: x[i] is position i - 3 counted from the first output (an even position), y the
+// outputs.  Every update has the value of the step-by-step scheme over the whole line.  A
+// thread per eight outputs repeats 6 of 22 (9/7) or 1 of 9 (5/3) updates of its neighbours, but
+// the chain is four updates long; one thread per line streamed 72 samples through shared
+// memory one after the other (a 64x64 tile's two passes took 4 us of latency).
+constexpr int SEG = 8, SEG_IN = SEG + 7;
 template <bool REV>
-__device__ __forceinline__ void lift_line(typename DwtTypes<REV>::T *p, int st) {
-  constexpr int NP = DWT_N / 2;  // 36 pairs
+__device__ __forceinline__ void lift_segment(const typename DwtTypes<REV>::T *x, typename DwtTypes<REV>::T *y) {
   if constexpr (REV) {
     // x[2n] -= (x[2n-1] + x[2n+1] + 2) >> 2; x[2n+1] += (x[2n] + x[2n+2]) >> 1
-    int xo_prev = p[st], e_prev = p[0];  // pair 0: x[0] is not updated
-#pragma unroll 5
-    for (int m = 1; m < NP; ++m) {
-      const int xe = p[2 * m * st], xo = p[(2 * m + 1) * st];
-      const int e = xe - ((xo_prev + xo + 2) >> 2);
-      const int o = xo_prev + ((e_prev + e) >> 1);  // position 2m-1
-      p[2 * m * st] = e;
-      p[(2 * m - 1) * st] = o;
-      xo_prev = xo;
-      e_prev = e;
+    int ev[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) ev[k] = x[2 * k + 3] - ((x[2 * k + 2] + x[2 * k + 4] + 2) >> 2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      y[2 * k] = ev[k];
+      y[2 * k + 1] = x[2 * k + 4] + ((ev[k] + ev[k + 1]) >> 1);
     }
   } else {
     // steps c0 (evens), c1 (odds), c2 (evens), c3 (odds): x -= c * (left + right), each
     // operation rounded separately
     const float c0 = 0.44350685204397f, c1 = 0.88291107553093f, c2 = -0.05298011857296f, c3 = -1.58613434205992f;
-    const float x0 = p[0], x1 = p[st];
-    const float x2 = p[2 * st], x3 = p[3 * st];
-    // m = 1
-    float e0_prev = lift97(x2, c0, x1, x3);     // e0 at 2
-    float o1_prev = lift97(x1, c1, x0, e0_prev);  // o1 at 1 (e0 at 0 = x0)
-    float e2_prev = x0;                            // e2 at 0 = x0
-    float xo_prev = x3;
-    p[0] = x0;
-#pragma unroll 5
-    for (int m = 2; m < NP; ++m) {
-      const float xe = p[2 * m * st], xo = p[(2 * m + 1) * st];
-      const float e0 = lift97(xe, c0, xo_prev, xo);           // position 2m
-      const float o1 = lift97(xo_prev, c1, e0_prev, e0);      // position 2m-1
-      const float e2 = lift97(e0_prev, c2, o1_prev, o1);      // position 2m-2
-      const float o3 = lift97(o1_prev, c3, e2_prev, e2);      // position 2m-3
-      p[(2 * m - 2) * st] = e2;
-      p[(2 * m - 3) * st] = o3;
-      xo_prev = xo;
-      e0_prev = e0;
-      o1_prev = o1;
-      e2_prev = e2;
+    float e0[7], o1[6], e2[5];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) e0[k] = lift97(x[2 * k + 1], c0, x[2 * k], x[2 * k + 2]);  // positions -2 .. 10
+#pragma unroll
+    for (int k = 0; k < 6; ++k) o1[k] = lift97(x[2 * k + 2], c1, e0[k], e0[k + 1]);  // -1 .. 9
+#pragma unroll
+    for (int k = 0; k < 5; ++k) e2[k] = lift97(e0[k + 1], c2, o1[k], o1[k + 1]);  // 0 .. 8
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      y[2 * k] = e2[k];
+      y[2 * k + 1] = lift97(o1[k + 1], c3, e2[k], e2[k + 1]);  // 1 .. 7
     }
   }
 }
@@ -158,13 +158,21 @@ __device__ __forceinline__ typename DwtTypes<REV>::T *dwt_buf(int id, void *a, v
   return (T *)(id == 0 ? a : (id == 1 ? b : c));
 }
 
-// Shared memory of one CTA: the staged window, the reference-compat column-end inputs and
-// the source row / column of every window line (mirrored, low or high part)
-template <bool REV>
+// Shared memory of one window of a TxT output tile: the staged samples and the
+// reference-compat column-end inputs.  Odd pitch: conflict-free column access.
+template <bool REV, int TILE = DWT_T>
 struct DwtSmem {
-  typename DwtTypes<REV>::T tile[DWT_N * DWT_PITCH];
-  typename DwtTypes<REV>::T keep[2][DWT_T];
-  int32_t srow[DWT_N], scol[DWT_N];
+  static constexpr int N = TILE + 2 * DWT_H, PITCH = N + 1;
+  typename DwtTypes<REV>::T tile[N * PITCH];
+  typename DwtTypes<REV>::T keep[2][TILE];
+};
+// The rows of a level kernel's window after the row pass, in a buffer of their own: no thread
+// holds its outputs while others still read (41 KB a CTA, five CTAs an SM)
+template <bool REV, int TILE = DWT_T>
+struct LevelSmem {
+  static constexpr int MID_PITCH = TILE + 1;
+  DwtSmem<REV, TILE> win;
+  typename DwtTypes<REV>::T mid[DwtSmem<REV, TILE>::N * MID_PITCH];
 };
 
 // Inputs of one window: the level's Mallat quadrants (`quad`) and the LL quadrant
@@ -177,135 +185,228 @@ struct WinSrc {
   int stride_ll;
 };
 
-// Rebuild the 64x64 output tile at (ox, oy) of one level for `nw` windows of the same
-// geometry (the components of one tile at their last level, or one tile-component): the
-// results are left in the centre of each window, S[w].tile[(y + 4) * DWT_PITCH + x + 4].
-template <bool REV>
-__device__ __forceinline__ void dwt_windows(DwtSmem<REV> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
-                                            int lh, bool ll_gain, float gain, bool refcompat, int ox, int oy) {
+// Stage the window of the tile at (ox, oy) with asynchronous 4-byte copies: every thread issues
+// all of its loads before waiting.  A warp copies a window row: lane l holds positions l,
+// l + 32 and l + 64 (as far as the row goes), even ones from the low part and odd ones from the
+// high part of the line (64 contiguous bytes of each per copy).  The mirror keeps the parity
+// and the warps' number is even, so a lane's part and a warp's row part never change: inside the
+// level a warp's pointers advance by whole lines.
+template <bool REV, int TILE>
+__device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
+                                          int lh, int ox, int oy) {
   typedef typename DwtTypes<REV>::T T;
-  // source line of every window row / column: window index i <-> position o - 4 + i, whose
-  // mirror keeps its parity, so even window lines come from the low part and odd ones
-  // from the high part (the same for every window)
-  for (int i = threadIdx.x; i < 2 * DWT_N; i += blockDim.x) {
-    const bool col = i >= DWT_N;
-    const int w = col ? i - DWT_N : i;
-    const int n = col ? rw : rh, lo = col ? lw : lh;
-    // the window may reach far past a level smaller than the tile: full periodic mirror
-    const int x = mirror((col ? ox : oy) - DWT_H + w, n);
-    const int sl = (x & 1) ? lo + (x >> 1) : (x >> 1);
-    if (col) S[0].scol[w] = sl;
-    else S[0].srow[w] = sl;
-  }
-  __syncthreads();
-  // stage quadrant by quadrant with asynchronous 4-byte copies (cp.async): every thread
-  // issues all of its loads before waiting, so a CTA has all its windows in flight;
-  // consecutive threads read consecutive source columns
-  constexpr int QN = DWT_N / 2;  // 36 window lines of each parity
-  // a warp copies one quadrant row at a time; each lane holds the source columns of
-  // quadrant columns j = lane and (lanes 0..3) j = lane + 32, for both parities
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  const bool two = lane < QN - 32;
-  const int sc_e0 = S[0].scol[2 * lane], sc_o0 = S[0].scol[2 * lane + 1];
-  const int sc_e1 = two ? S[0].scol[2 * (lane + 32)] : 0, sc_o1 = two ? S[0].scol[2 * (lane + 32) + 1] : 0;
-  for (int w = 0; w < nw; ++w) {
-    const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(S[w].tile);
+  constexpr int N = DwtSmem<REV, TILE>::N, PITCH = DwtSmem<REV, TILE>::PITCH, COLS = (N + 31) / 32;
+  constexpr int WARPS = DWT_THREADS / 32;
+  static_assert(DWT_THREADS == FUSED_THREADS && WARPS % 2 == 0 && N % WARPS == 0, "rows are dealt to an even number of warps");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int odd = lane & 1, high = warp & 1;
+  int col[COLS];
 #pragma unroll
-    for (int qd = 0; qd < 4; ++qd) {  // quadrant LL, HL, LH, HH
-      const T *qbase = qd == 0 ? src[w].llsrc : src[w].quad;
-      const int qstride = qd == 0 ? src[w].stride_ll : src[w].stride_q;
-      const int odd = qd & 1;
-      const T *lo0 = qbase + (odd ? sc_o0 : sc_e0), *lo1 = qbase + (odd ? sc_o1 : sc_e1);
-      const uint32_t d0 = tile_s + 4u * (odd + 2 * lane), d1 = d0 + 4u * 64;
-#pragma unroll 2
-      for (int r = warp; r < QN; r += nwarps) {
-        const int iy = 2 * r + (qd >> 1);
-        const size_t row = (size_t)S[0].srow[iy] * qstride;
-        const uint32_t drow = 4u * iy * DWT_PITCH;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d0 + drow), "l"(lo0 + row));
-        if (two) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d1 + drow), "l"(lo1 + row));
-      }
+  for (int j = 0; j < COLS; ++j) col[j] = (mirror(ox - DWT_H + lane + 32 * j, rw) >> 1) + (odd ? lw : 0);
+  const bool last = lane < N - 32 * (COLS - 1);
+  const bool inside = oy >= DWT_H && oy + TILE + DWT_H <= rh;
+  for (int w = 0; w < nw; ++w) {
+    const bool ll = !high && !odd;
+    const T *base = ll ? src[w].llsrc : src[w].quad + (high ? (size_t)lh * src[w].stride_q : 0);
+    const int stride = ll ? src[w].stride_ll : src[w].stride_q;
+    const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(S[w].tile + warp * PITCH + lane);
+    auto copy = [&](const T *line, uint32_t d) {
+#pragma unroll
+      for (int j = 0; j < COLS; ++j)
+        if (j < COLS - 1 || last)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 128 * j), "l"(line + col[j]));
+    };
+    if (inside) {
+      const T *line = base + (size_t)((oy - DWT_H + warp) >> 1) * stride;
+      const size_t step = (size_t)(WARPS / 2) * stride;
+#pragma unroll
+      for (int i = 0; i < N / WARPS; ++i, line += step) copy(line, d0 + 4 * PITCH * WARPS * i);
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < N / WARPS; ++i)
+        copy(base + (size_t)(mirror(oy - DWT_H + warp + WARPS * i, rh) >> 1) * stride, d0 + 4 * PITCH * WARPS * i);
     }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-  if (!REV && ll_gain) {
-    // the reconstructed LL entering a finer 9/7 level is scaled by K_lo^2
-    for (int e = threadIdx.x; e < nw * QN * QN; e += blockDim.x) {
-      const int w = e / (QN * QN), q = e - w * QN * QN, r = q / QN, j = q - r * QN;
-      T *v = S[w].tile + 2 * r * DWT_PITCH + 2 * j;
-      *v = (T)__fmul_rn((float)*v, gain);
+}
+
+// Rebuild the TILE x TILE output tile at (ox, oy) of one level for `nw` windows of the same
+// geometry (the components of one tile at their last level, or one tile-component).  The
+// results are left in the centre of each window, S[w].tile[(y + 4) * PITCH + x + 4], or
+// (DIRECT: a single window, its rows in `mid`) stored to `out` from the column pass.
+template <bool REV, bool DIRECT, int TILE>
+__device__ __forceinline__ void dwt_windows(DwtSmem<REV, TILE> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
+                                            int lh, bool ll_gain, float gain, bool refcompat, int ox, int oy,
+                                            typename DwtTypes<REV>::T *mid, typename DwtTypes<REV>::T *out,
+                                            int stride_out) {
+  typedef typename DwtTypes<REV>::T T;
+  constexpr int N = DwtSmem<REV, TILE>::N, PITCH = DwtSmem<REV, TILE>::PITCH, MID_PITCH = TILE + 1;
+  dwt_stage<REV, TILE>(S, nw, src, rw, rh, lw, lh, ox, oy);
+  // Rows: a thread lifts eight outputs of a row; consecutive threads take consecutive rows (the
+  // odd pitch keeps the banks apart).  The reconstructed LL entering a finer 9/7 level is
+  // scaled by K_lo^2 on the way.
+  constexpr int SEGS = TILE / SEG, ROW_TASKS = N * SEGS;
+  constexpr int RT = (ROW_TASKS + DWT_THREADS - 1) / DWT_THREADS;
+  auto row_task = [&](int w, int seg, int r, T *y) {
+    const T *p = S[w].tile + r * PITCH + SEG * seg + DWT_H - 3;
+    T x[SEG_IN];
+#pragma unroll
+    for (int k = 0; k < SEG_IN; ++k) x[k] = p[k];
+    if constexpr (!REV) {
+      if (ll_gain) {
+        const float g = !(r & 1) ? gain : 1.f;
+#pragma unroll
+        for (int k = 1; k < SEG_IN; k += 2) x[k] = __fmul_rn(x[k], g);
+      }
     }
-    __syncthreads();
-  }
-  if (rw > 1) {
-    for (int l = threadIdx.x; l < nw * DWT_N; l += blockDim.x) {
-      const int w = l / DWT_N, r = l - w * DWT_N;
-      lift_line<REV>(S[w].tile + r * DWT_PITCH, 1);
+    if (rw > 1) {
+      lift_segment<REV>(x, y);
+    } else {
+#pragma unroll
+      for (int k = 0; k < SEG; ++k) y[k] = x[k + 3];
     }
-    __syncthreads();
+  };
+  if (DIRECT) {
+#pragma unroll 1
+    for (int t = threadIdx.x; t < ROW_TASKS; t += DWT_THREADS) {
+      const int seg = t / N, r = t - seg * N;
+      T y[SEG];
+      row_task(0, seg, r, y);
+      T *p = mid + r * MID_PITCH + SEG * seg;
+#pragma unroll
+      for (int k = 0; k < SEG; ++k) p[k] = y[k];
+    }
+  } else {
+    // in place: the outputs wait in registers until the window's inputs have been read
+    for (int w = 0; w < nw; ++w) {
+      T y[RT][SEG];
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const int t = threadIdx.x + i * DWT_THREADS;
+        if (t < ROW_TASKS) row_task(w, t / N, t % N, y[i]);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const int t = threadIdx.x + i * DWT_THREADS;
+        if (t < ROW_TASKS) {
+          T *p = S[w].tile + (t % N) * PITCH + SEG * (t / N) + DWT_H;
+#pragma unroll
+          for (int k = 0; k < SEG; ++k) p[k] = y[i][k];
+        }
+      }
+    }
   }
+  __syncthreads();
   // reference-compat: keep the horizontally transformed inputs the column end reads
   const int n = rh;
-  const bool fix = REV && refcompat && n >= 3 && (oy <= n - 1) && (n - 2 < oy + DWT_T);
-  int rowA = -1, rowB = -1;
+  const bool fix = REV && refcompat && n >= 3 && (oy <= n - 1) && (n - 2 < oy + TILE);
   if (fix) {
-    if (!(n & 1)) {
-      rowA = n - 3;  // H[m-2]
-    } else {
+    int rowA = n - 3, rowB = -1;  // H[m-2]
+    if (n & 1) {
       const int m = (n + 1) / 2;
       rowA = n - 3;                 // L[m-2]
       rowB = (m >= 3) ? n - 4 : 1;  // H[m-3] (H[0] when m == 2)
     }
-    for (int e = threadIdx.x; e < nw * DWT_T; e += blockDim.x) {
-      const int w = e / DWT_T, c = e - w * DWT_T;
-      S[w].keep[0][c] = S[w].tile[(rowA - oy + DWT_H) * DWT_PITCH + DWT_H + c];
-      if (rowB >= 0) S[w].keep[1][c] = S[w].tile[(rowB - oy + DWT_H) * DWT_PITCH + DWT_H + c];
+    for (int e = threadIdx.x; e < nw * TILE; e += blockDim.x) {
+      const int w = e / TILE, c = e - w * TILE;
+      const T *rows = DIRECT ? mid + c : S[w].tile + DWT_H + c;
+      constexpr int pitch = DIRECT ? MID_PITCH : PITCH;
+      S[w].keep[0][c] = rows[(rowA - oy + DWT_H) * pitch];
+      if (rowB >= 0) S[w].keep[1][c] = rows[(rowB - oy + DWT_H) * pitch];
     }
-    __syncthreads();
   }
-  if (rh > 1) {
-    for (int l = threadIdx.x; l < nw * DWT_T; l += blockDim.x) {
-      const int w = l / DWT_T, c = l - w * DWT_T;
-      lift_line<REV>(S[w].tile + DWT_H + c, DWT_PITCH);
+  // Columns: a thread lifts eight outputs of a column, consecutive threads consecutive columns
+  constexpr int COL_TASKS = TILE * SEGS, CT = (COL_TASKS + DWT_THREADS - 1) / DWT_THREADS, STEP = DWT_THREADS / TILE;
+  const int ow = min(TILE, rw - ox), oh = min(TILE, rh - oy);
+  auto col_task = [&](const T *p, int pitch, T *y) {
+    T x[SEG_IN];
+#pragma unroll
+    for (int k = 0; k < SEG_IN; ++k) x[k] = p[k * pitch];
+    if (rh > 1) {
+      lift_segment<REV>(x, y);
+    } else {
+#pragma unroll
+      for (int k = 0; k < SEG; ++k) y[k] = x[k + 3];
     }
-    __syncthreads();
+  };
+  const int c = threadIdx.x % TILE;
+  if (DIRECT) {
+#pragma unroll 1
+    for (int seg = threadIdx.x / TILE; seg < SEGS; seg += STEP) {
+      T y[SEG];
+      col_task(mid + (SEG * seg + DWT_H - 3) * MID_PITCH + c, MID_PITCH, y);
+      if (!fix) {
+        T *o = out + (size_t)(oy + SEG * seg) * stride_out + ox + c;
+        const int rows = c < ow ? oh - SEG * seg : 0;
+        if (rows >= SEG) {
+#pragma unroll
+          for (int k = 0; k < SEG; ++k, o += stride_out) *o = y[k];
+        } else {
+#pragma unroll
+          for (int k = 0; k < SEG; ++k, o += stride_out)
+            if (k < rows) *o = y[k];
+        }
+      } else {
+        T *p = S[0].tile + (SEG * seg + DWT_H) * PITCH + DWT_H + c;
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) p[k * PITCH] = y[k];
+      }
+    }
+    if (!fix) return;
+  } else {
+    for (int w = 0; w < nw; ++w) {
+      T y[CT][SEG];
+#pragma unroll
+      for (int i = 0; i < CT; ++i)
+        col_task(S[w].tile + (SEG * (threadIdx.x / TILE + i * STEP) + DWT_H - 3) * PITCH + DWT_H + c, PITCH, y[i]);
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < CT; ++i) {
+        T *p = S[w].tile + (SEG * (threadIdx.x / TILE + i * STEP) + DWT_H) * PITCH + DWT_H + c;
+#pragma unroll
+        for (int k = 0; k < SEG; ++k) p[k * PITCH] = y[i][k];
+      }
+    }
   }
+  __syncthreads();
   if constexpr (REV) {
     if (fix) {
-      for (int e = threadIdx.x; e < nw * DWT_T; e += blockDim.x) {
-        const int w = e / DWT_T, c = e - w * DWT_T;
-        T *col = S[w].tile + DWT_H + c;
+      for (int e = threadIdx.x; e < nw * TILE; e += blockDim.x) {
+        const int w = e / TILE, cc = e - w * TILE;
+        T *colp = S[w].tile + DWT_H + cc;
         const int r1 = n - 1 - oy + DWT_H, r2 = n - 2 - oy + DWT_H, r3 = n - 3 - oy + DWT_H;
         if (!(n & 1)) {
-          col[r1 * DWT_PITCH] = S[w].keep[0][c] + col[r2 * DWT_PITCH];
+          colp[r1 * PITCH] = S[w].keep[0][cc] + colp[r2 * PITCH];
         } else {
-          const T hx = S[w].keep[1][c];
-          const T x1 = S[w].keep[0][c] - ((hx + 1) >> 1);
-          col[r1 * DWT_PITCH] = x1;
-          col[r2 * DWT_PITCH] = hx + ((x1 + col[r3 * DWT_PITCH]) >> 1);
+          const T hx = S[w].keep[1][cc];
+          const T x1 = S[w].keep[0][cc] - ((hx + 1) >> 1);
+          colp[r1 * PITCH] = x1;
+          colp[r2 * PITCH] = hx + ((x1 + colp[r3 * PITCH]) >> 1);
         }
       }
       __syncthreads();
     }
   }
+  if (DIRECT) {
+    for (int i = threadIdx.x; i < TILE * TILE; i += blockDim.x) {
+      const int yy = i / TILE, xx = i % TILE;
+      if (yy < oh && xx < ow)
+        out[(size_t)(oy + yy) * stride_out + ox + xx] = S[0].tile[(yy + DWT_H) * PITCH + xx + DWT_H];
+    }
+  }
 }
 
-// One 64x64 output tile of one level of one tile-component, stored to `out`.
-template <bool REV>
-__device__ __forceinline__ void dwt_tile(DwtSmem<REV> &S, const typename DwtTypes<REV>::T *quad, int stride_q,
+// One output tile of one level of one tile-component, stored to `out`.
+template <bool REV, int TILE>
+__device__ __forceinline__ void dwt_tile(LevelSmem<REV, TILE> &S, const typename DwtTypes<REV>::T *quad, int stride_q,
                                          const typename DwtTypes<REV>::T *llsrc, int stride_ll,
                                          typename DwtTypes<REV>::T *out, int stride_out, int rw, int rh, int lw,
                                          int lh, bool ll_gain, float gain, bool refcompat, int ox, int oy) {
   const WinSrc<REV> src{quad, stride_q, llsrc, stride_ll};
-  dwt_windows<REV>(&S, 1, &src, rw, rh, lw, lh, ll_gain, gain, refcompat, ox, oy);
-  const int ow = min(DWT_T, rw - ox), oh = min(DWT_T, rh - oy);
-  for (int i = threadIdx.x; i < DWT_T * DWT_T; i += blockDim.x) {
-    const int yy = i / DWT_T, xx = i % DWT_T;
-    if (yy < oh && xx < ow)
-      out[(size_t)(oy + yy) * stride_out + ox + xx] = S.tile[(yy + DWT_H) * DWT_PITCH + xx + DWT_H];
-  }
-  __syncthreads();
+  dwt_windows<REV, true, TILE>(&S.win, 1, &src, rw, rh, lw, lh, ll_gain, gain, refcompat, ox, oy, S.mid, out, stride_out);
+  __syncthreads();  // the window is free for the next tile
 }
 
 template <bool REV>
@@ -313,14 +414,14 @@ __global__ void __launch_bounds__(DWT_THREADS) dwt_level_kernel(const DwtLevel *
                                                         const DwtTask *__restrict__ tasks, int ntasks, void *bufA,
                                                         void *bufB, void *bufC, float ll_gain_value) {
   typedef typename DwtTypes<REV>::T T;
-  __shared__ DwtSmem<REV> S;
+  __shared__ LevelSmem<REV> S;
   for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
     const DwtTask tk = tasks[task];
     const DwtLevel L = levels[tk.level];
     const T *A = dwt_buf<REV>(0, bufA, bufB, bufC) + L.base;
     const T *LLsrc = dwt_buf<REV>(L.ll_src, bufA, bufB, bufC) + L.base;
     T *out = dwt_buf<REV>(L.out_dst, bufA, bufB, bufC) + L.base;
-    dwt_tile<REV>(S, A, L.stride, LLsrc, L.stride, out, L.stride, L.rw, L.rh, L.lw, L.lh, L.ll_gain != 0,
+    dwt_tile<REV, DWT_T>(S, A, L.stride, LLsrc, L.stride, out, L.stride, L.rw, L.rh, L.lw, L.lh, L.ll_gain != 0,
                   ll_gain_value, L.refcompat != 0, tk.tx * DWT_T, tk.ty * DWT_T);
   }
 }
@@ -476,7 +577,7 @@ __global__ void __launch_bounds__(256) output_kernel(const OutGroup *__restrict_
 // inverse MCT reads the components' windows in shared memory): one CTA per 64x64 tile.
 // Dynamic shared memory: `nwin` DwtSmem windows.
 template <bool REV>
-__global__ void __launch_bounds__(FUSED_THREADS) last_level_output_kernel(const FusedGroup *__restrict__ groups,
+__global__ void __launch_bounds__(FUSED_THREADS, 3) last_level_output_kernel(const FusedGroup *__restrict__ groups,
                                                                         const OutTask *__restrict__ tasks, int ntasks,
                                                                         void *bufA, void *bufB, void *bufC,
                                                                         float ll_gain_value, uint8_t *out) {
@@ -496,7 +597,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) last_level_output_kernel(const 
       have[c] = true;
     }
     const int ox = tk.tx * DWT_T, oy = tk.ty * DWT_T;
-    dwt_windows<REV>(S, nc, src, F.rw, F.rh, F.lw, F.lh, F.ll_gain != 0, ll_gain_value, F.refcompat != 0, ox, oy);
+    dwt_windows<REV, false, DWT_T>(S, nc, src, F.rw, F.rh, F.lw, F.lh, F.ll_gain != 0, ll_gain_value, F.refcompat != 0, ox, oy,
+                            nullptr, nullptr, 0);
     const int ow = min(DWT_T, F.rw - ox), oh = min(DWT_T, F.rh - oy);
     if (G.fmt == 2 && G.bitdepth == 8 && G.mct && nc == 3) {
       // 24-bit RGB after the inverse MCT (the common path): sixteen pixels per thread (48
@@ -677,18 +779,45 @@ __global__ void __launch_bounds__(128) dwt_coarse_kernel(const CoarseTask *__res
 
 namespace j2k_dev {
 
-// One level of one tile-component with every buffer given explicitly (no descriptor
-// tables in device memory): the CTA index selects the 64x64 output tile.  Used by the
-// entry point that runs on a static scratch array (noalloc.cu).
+// Every level of one tile-component in one cooperative launch, all buffers given explicitly (no
+// descriptor tables in device memory); CTAs take the 64x64 output tiles of a level in turn and
+// meet at a grid-wide barrier between levels.  Used by the entry point that runs on a static
+// scratch array (noalloc.cu), whose levels are mostly small: a launch each cost 5 to 6 us.
 template <bool REV>
-__global__ void __launch_bounds__(DWT_THREADS) dwt_level_explicit_kernel(
-    const typename DwtTypes<REV>::T *__restrict__ quad, int stride_q, const typename DwtTypes<REV>::T *llsrc,
-    int stride_ll, typename DwtTypes<REV>::T *out, int stride_out, int rw, int rh, int lw, int lh, int ll_gain,
-    float ll_gain_value, int refcompat) {
-  __shared__ DwtSmem<REV> S;
-  const int tiles_x = (rw + DWT_T - 1) / DWT_T;
-  dwt_tile<REV>(S, quad, stride_q, llsrc, stride_ll, out, stride_out, rw, rh, lw, lh, ll_gain != 0, ll_gain_value,
-                refcompat != 0, (blockIdx.x % tiles_x) * DWT_T, (blockIdx.x / tiles_x) * DWT_T);
+struct AllLevels {
+  typedef typename DwtTypes<REV>::T T;
+  const T *coef;  // Mallat layout, row stride coef_stride
+  T *half[2];     // intermediate resolutions (level r to half[r & 1]), row stride half_stride
+  T *out;
+  int coef_stride, half_stride, out_stride, levels, refcompat;
+  float ll_gain;
+  int res_w[J2K_MAX_LEVELS + 1], res_h[J2K_MAX_LEVELS + 1];
+};
+// A level that 64x64 tiles would spread over less than half of the CTAs is cut into 32x32 tiles:
+// more of the chip works on it, each CTA for a shorter time.
+constexpr int SMALL_T = 32;
+template <bool REV>
+__global__ void __launch_bounds__(DWT_THREADS) dwt_all_levels_kernel(const AllLevels<REV> L) {
+  typedef typename DwtTypes<REV>::T T;
+  __shared__ __align__(16) uint8_t smem[sizeof(LevelSmem<REV, DWT_T>)];
+  for (int r = 1; r <= L.levels; ++r) {
+    const int rw = L.res_w[r], rh = L.res_h[r], lw = L.res_w[r - 1], lh = L.res_h[r - 1];
+    const T *ll = r == 1 ? L.coef : L.half[(r - 1) & 1];
+    const int ll_stride = r == 1 ? L.coef_stride : L.half_stride;
+    T *dst = r == L.levels ? L.out : L.half[r & 1];
+    const int dst_stride = r == L.levels ? L.out_stride : L.half_stride;
+    auto level = [&](auto edge) {
+      constexpr int E = decltype(edge)::value;
+      const int tiles_x = (rw + E - 1) / E, tiles = tiles_x * ((rh + E - 1) / E);
+      for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+        dwt_tile<REV, E>(*reinterpret_cast<LevelSmem<REV, E> *>(smem), L.coef, L.coef_stride, ll, ll_stride, dst, dst_stride,
+                         rw, rh, lw, lh, !REV && r > 1, L.ll_gain, L.refcompat != 0, (t % tiles_x) * E, (t / tiles_x) * E);
+    };
+    const int large = ((rw + DWT_T - 1) / DWT_T) * ((rh + DWT_T - 1) / DWT_T);
+    if (2 * large <= (int)gridDim.x) level(std::integral_constant<int, SMALL_T>{});
+    else level(std::integral_constant<int, DWT_T>{});
+    if (r < L.levels) cooperative_groups::this_grid().sync();
+  }
 }
 
 }  // namespace j2k_dev
