@@ -70,7 +70,7 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
   for (int i = threadIdx.x; i < (int)(sizeof(T1Tables) / 16); i += blockDim.x)
     reinterpret_cast<uint4 *>(smem)[i] = reinterpret_cast<const uint4 *>(&g_t1tables)[i];
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = LATENCY ? 0 : threadIdx.x >> 5, lane = LATENCY ? threadIdx.x : threadIdx.x & 31;
   uint8_t *mine = smem + sizeof(T1Tables) + warp * Lay::PER_WARP;
   Block b;
   b.rf = reinterpret_cast<uint4 *>(mine + Lay::RF);
@@ -129,7 +129,9 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
 
 // The two kernel forms.  The throughput (compact) form keeps the default register target,
 // which leaves room for 32 resident warps per SM; the latency form (batches that fit about two
-// waves) may use more registers, as occupancy does not bound it.
+// waves) may use more registers, as occupancy does not bound it, and has one warp a CTA: its
+// shared-memory addresses are constants then (one 2048x2048 RGB 9/7 picture 3.86 -> 3.63 ms, one
+// 256x256 picture 1.14 -> 1.04 ms against CTAs of eight warps).
 #define J2K_T1_PARAMS                                                                                   \
   const j2k_cblk *__restrict__ cbs, const uint32_t *__restrict__ order, int n, int *__restrict__ counter, \
       const uint8_t *__restrict__ bytes, const uint32_t *__restrict__ seglens, void *__restrict__ coef,   \
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(256) t1_kernel_compact(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, false>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 template <int MAXW, int MAXH>
-__global__ void __launch_bounds__(256, 1) t1_kernel_latency(J2K_T1_PARAMS) {
+__global__ void __launch_bounds__(32, 16) t1_kernel_latency(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, true>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 #undef J2K_T1_PARAMS
@@ -430,9 +432,9 @@ void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, c
   typedef T1Layout<MAXW, MAXH> Lay;
   int best_w = 1, best_ctas = 1, best_warps = 0;
   // a queue shorter than the resident warps is spread over all SMs: its time is that of its
-  // longest blocks, which two warps of one scheduler would lengthen
+  // longest blocks, which two warps of one scheduler would lengthen (the latency form always is)
   const int spread = std::max(1, (n + c->sm_count - 1) / c->sm_count);
-  const int wmax = std::min(spread, warps_per_cta > 0 ? std::min(8, warps_per_cta) : 8);
+  const int wmax = LATENCY ? 1 : std::min(spread, warps_per_cta > 0 ? std::min(8, warps_per_cta) : 8);
   for (int w = 1; w <= wmax; ++w) {
     const size_t sm = sizeof(T1Tables) + (size_t)w * Lay::PER_WARP;
     if (sm > c->smem_optin) break;

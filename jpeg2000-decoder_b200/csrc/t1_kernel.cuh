@@ -204,20 +204,24 @@ __device__ __forceinline__ uint32_t mq_symbol(Mq &m, uint8_t *slot, uint2 &e, co
   m.l0 = __funnelshift_l(m.l1, m.l0, n);
   m.l1 <<= n;
   m.T -= n;
+  if (!LATENCY && m.T < T_MIN) mq_refill(m);  // else before the symbol, once for two of them
   return mps ^ (uint32_t)lps;
 }
-// Before a pair of symbols / between the two (a refill is due there only while a carry waits)
+// Before a pair of symbols / between the two (a refill is due there only while a carry waits).
+// The throughput form looks after every renormalisation instead: its common symbol has none.
+template <bool LATENCY>
 __device__ __forceinline__ void mq_ready(Mq &m) {
-  if (m.T < T_MIN) mq_refill(m);
+  if (LATENCY && m.T < T_MIN) mq_refill(m);
 }
+template <bool LATENCY>
 __device__ __forceinline__ void mq_level(Mq &m) {
-  if (m.T < 0) mq_refill(m);
+  if (LATENCY && m.T < 0) mq_refill(m);
 }
 // a symbol on its own
 template <bool LATENCY>
 __device__ __forceinline__ uint32_t mq_decode(Mq &m, uint8_t *cx, uint32_t off, const uint8_t *tab) {
   uint2 e = *reinterpret_cast<const uint2 *>(cx + off);
-  mq_ready(m);
+  mq_ready<LATENCY>(m);
   return mq_symbol<LATENCY>(m, cx + off, e, tab);
 }
 
@@ -479,6 +483,7 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
         const int bit = __ffs(live) - 1;
         uint32_t *wp = row + c0 + bit;
         uint32_t W = *wp, x, k3 = 0;
+        const uint32_t L = wp[-1], R = wp[1];  // their own bits do not change during the walk of this column
         bool forced = false;
         if (PASS == P_CLEANUP && ((zero >> bit) & 1)) {
           uint2 e = *reinterpret_cast<const uint2 *>(b.cx + RUN_OFF);
@@ -493,7 +498,7 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
             continue;
           }
           live &= live - 1;
-          mq_ready(mq);
+          mq_ready<LATENCY>(mq);
           if (!mq_symbol<LATENCY>(mq, b.cx + RUN_OFF, e, b.mq)) continue;
           k3 = mq_decode<LATENCY>(mq, b.cx, UNI_OFF, b.mq) * 6;
           k3 += mq_decode<LATENCY>(mq, b.cx, UNI_OFF, b.mq) * 3;
@@ -515,7 +520,7 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
             } else {
               const uint32_t off = b.zc[(W >> k3) & 0x1EF];
               uint2 e = *reinterpret_cast<const uint2 *>(b.cx + off);
-              mq_ready(mq);
+              mq_ready<LATENCY>(mq);
               d = mq_symbol<LATENCY>(mq, b.cx + off, e, b.mq);
             }
             if (!d) continue;
@@ -526,9 +531,9 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
           if (RAW) {
             sign = raw_bit(raw);
           } else {
-            const uint32_t sv = b.sc[sign_index(W, wp[-1], wp[1], k3)], off = sv & 0xF8;
+            const uint32_t sv = b.sc[LATENCY ? sign_index(W, L, R, k3) : sign_index(W, wp[-1], wp[1], k3)], off = sv & 0xF8;
             uint2 e = *reinterpret_cast<const uint2 *>(b.cx + off);
-            mq_level(mq);
+            mq_level<LATENCY>(mq);
             sign = mq_symbol<LATENCY>(mq, b.cx + off, e, b.mq) ^ (sv & 1);
           }
           hit = 0xffffffffu;

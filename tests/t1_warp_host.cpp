@@ -259,10 +259,10 @@ extern "C" int t1_warp_host_symbols(uint32_t seed, int n, int cut, int latency, 
     wrong += (latency ? mq_symbol<true>(m, slot, e, tab) : mq_symbol<false>(m, slot, e, tab)) != sym[i];
   };
   for (int i = 0; i < n;) {
-    mq_ready(m);
+    if (latency) mq_ready<true>(m);
     one(i++);
     if (i % cut == 0 || i >= n) continue;
-    mq_level(m);
+    if (latency) mq_level<true>(m);
     one(i++);
   }
   return wrong;
