@@ -38,7 +38,7 @@ struct Slot {
   DecodeJobConfig cfg;
   CodeStreamProperties props{};
   std::vector<uint8_t> codestream;
-  std::vector<uint8_t> result, thumb;
+  j2k::ByteBuffer result, thumb;  // filled by the copy from the device, not cleared before it
   std::vector<int32_t> comp_int;
   std::vector<float> comp_float;
   int comp_loaded = -1;
@@ -324,7 +324,7 @@ class GpuDecoder : public Decoder {
         j2k_gpu_output_device(ctx_, s->gpu_slot, &d, &bytes);
         if (bytes) {
           s->result.resize(bytes);
-          j2k_gpu_output_copy(ctx_, s->gpu_slot, s->result.data(), bytes);
+          if (j2k_gpu_output_copy(ctx_, s->gpu_slot, s->result.data(), bytes) != J2K_OK) st = J2K_ERR_CUDA;
         }
         s->status = st == J2K_OK ? READY : DECODE_ERROR;
         s->comp_loaded = -1;
@@ -335,7 +335,7 @@ class GpuDecoder : public Decoder {
   }
 
   // decode the slot's codestream again with other options into `out`
-  bool decode_side(Slot &s, int discard, int fmt, std::vector<uint8_t> &out) {
+  bool decode_side(Slot &s, int discard, int fmt, j2k::ByteBuffer &out) {
     finish_pending();
     j2k_plan *p = nullptr;
     if (j2k_plan_create_mt(s.codestream.data(), s.codestream.size(), discard, 0, s.cfg.mIgnoreComponents, tier2_threads(),
@@ -349,6 +349,7 @@ class GpuDecoder : public Decoder {
               j2k_gpu_output_copy(ctx_, 0, out.data(), out.size()) == J2K_OK;
     j2k_plan_destroy(p);
     resident_ = INVALID;
+    if (!ok) out.clear();
     return ok;
   }
 
