@@ -157,7 +157,7 @@ typedef struct j2k_gpu_tuning {
   int t1_latency_waves;  /* auto form without an autotuned choice: latency form while code-blocks <=
                             this many x 32 warps x SMs, compact above */
   int dwt_coarse;        /* the coarse levels of each tile-component (resolutions up to 64 samples a
-                            side) in one shared-memory kernel: 0 default (on), 1 on, 2 off (one
+                            side) in one shared-memory kernel: 0 default (off), 1 on, 2 off (one
                             launch per level) */
 } j2k_gpu_tuning;
 int j2k_gpu_set_tuning(j2k_gpu_ctx *ctx, const j2k_gpu_tuning *t);

@@ -215,7 +215,7 @@ struct j2k_gpu_ctx {
     float t1_ms = 0;
   };
   std::map<int, TuneEntry> tune_table;
-  int dwt_auto = 0;  // autotuned coarse-level choice (1 on, 2 off) for dwt_coarse 0; 0 = not tuned (on)
+  int dwt_auto = 0;  // autotuned coarse-level choice (1 on, 2 off) for dwt_coarse 0; 0 = not tuned (off)
   int sm_count = 148;
   size_t smem_optin = 227 * 1024;
 };
@@ -535,7 +535,9 @@ extern "C" int j2k_gpu_batch_stage(j2k_gpu_ctx *c, void *user_stream) {
   std::vector<FusedGroup> fgroups;
   std::vector<OutTask> ftasks[2];  // fused last levels: [0] 9/7, [1] 5/3
   std::vector<CoarseTask> ctasks[2];  // coarse levels synthesised in shared memory: [0] 9/7, [1] 5/3
-  const bool coarse_on = c->tuning.dwt_coarse == 1 || (c->tuning.dwt_coarse == 0 && c->dwt_auto != 2);
+  // one launch per level unless asked for or tuned otherwise: 0.040 against 0.048 to 0.054 ms for a
+  // 256x256 RGB and a 512x512 gray picture, 0.788 against 0.808 ms for 32 1080p frames
+  const bool coarse_on = c->tuning.dwt_coarse == 1 || (c->tuning.dwt_coarse == 0 && c->dwt_auto == 1);
   const bool lane_split = c->tuning.t1_form == 3;  // queue classes for the lane form
   int fwin = 1;
   uint64_t byte_base = 0;

@@ -226,11 +226,11 @@ extern "C" int t1_warp_host_symbols(uint32_t seed, int n, int cut, int latency, 
       }
       if (A < q) A = q;
       else C += q;
-      e = rec[1];
+      e = rec[2];
     } else {
       if (A < q) C += q;
       else A = q;
-      e = rec[2];
+      e = rec[3];
     }
     do {
       A <<= 1;
@@ -256,7 +256,7 @@ extern "C" int t1_warp_host_symbols(uint32_t seed, int n, int cut, int latency, 
   auto one = [&](int i) {
     uint8_t *slot = cx + ctx[i] * SLOT;
     uint2 e = *reinterpret_cast<uint2 *>(slot);
-    wrong += (latency ? mq_symbol<true>(m, slot, e, tab) : mq_symbol<false>(m, slot, e, tab)) != sym[i];
+    wrong += is_one(latency ? mq_symbol<true>(m, slot, e, tab) : mq_symbol<false>(m, slot, e, tab)) != sym[i];
   };
   for (int i = 0; i < n;) {
     if (latency) mq_ready<true>(m);
