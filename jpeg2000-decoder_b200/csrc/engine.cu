@@ -19,7 +19,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cstring>
 #include <new>
@@ -32,6 +31,7 @@
 #include "bmi_engine.h"
 #include "codestream.h"
 #include "dwt_kernel.cuh"
+#include "host_copy.h"
 #include "t1_kernel.cuh"
 #include "t1_lanes.cuh"
 
@@ -188,7 +188,7 @@ struct j2k_gpu_ctx {
   // page-locked pieces of the threaded copy of a large picture into pageable memory (allocated by
   // the first one, freed with the context)
   uint8_t *h_bounce = nullptr;
-  cudaEvent_t bounce_ev[8] = {};
+  cudaEvent_t bounce_ev[j2k::COPY_THREADS] = {};
   std::mutex bounce_mu;
   bool launched = false, synced = false, staged = false;
   bool copies_pending = false;  // output copies enqueued behind the decode (ev[5] follows them)
@@ -1098,54 +1098,31 @@ extern "C" int j2k_gpu_output_device(const j2k_gpu_ctx *c, int slot, const void 
 }
 
 namespace {
-// Copy of a large picture into pageable memory.  The driver's copy into such memory runs on one
-// host thread, which takes the page faults of a fresh destination as well: 53 MB of a
-// 4096x2160 48-bit picture took 11.3 ms (4.7 GB/s).  Here a few threads each bring pieces into a
-// page-locked piece of their own and move them on, so the faults and the copies overlap (the
-// same picture: 2.6 ms).  Smaller pictures mostly land in memory that the allocator hands out
-// again without faults, where the driver's copy is as fast (12.6 MB: 0.65 against 0.52 ms).
-constexpr size_t BOUNCE_PIECE = (size_t)1 << 20, BOUNCE_FROM = (size_t)16 << 20;
-constexpr int BOUNCE_THREADS = 8;
+// Copy of a large picture into pageable memory (host_copy.h): each thread brings pieces into a
+// page-locked piece of its own and moves them on, so the page faults and the copies overlap
 int copy_to_pageable(j2k_gpu_ctx *c, const uint8_t *src, uint8_t *dst, size_t bytes) {
   std::lock_guard<std::mutex> lk(c->bounce_mu);
   if (!c->h_bounce) {
     for (auto &e : c->bounce_ev)
       if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     void *p = nullptr;
-    if (cudaMallocHost(&p, BOUNCE_PIECE * BOUNCE_THREADS) != cudaSuccess) {
+    if (cudaMallocHost(&p, j2k::COPY_PIECE * j2k::COPY_THREADS) != cudaSuccess) {
       cudaGetLastError();
       return J2K_ERR_NOMEM;
     }
     c->h_bounce = (uint8_t *)p;
   }
-  const size_t pieces = (bytes + BOUNCE_PIECE - 1) / BOUNCE_PIECE;
-  const unsigned cores = std::thread::hardware_concurrency();
-  const int n = (int)std::min<size_t>({(size_t)BOUNCE_THREADS, pieces, std::max<size_t>(1, cores)});
-  std::atomic<int> failed{0};
-  std::atomic<size_t> next{0};
-  auto work = [&](int t) {
-    uint8_t *mine = c->h_bounce + (size_t)t * BOUNCE_PIECE;
-    if (cudaSetDevice(c->device) != cudaSuccess) failed = 1;
-    for (size_t k; !failed && (k = next.fetch_add(1)) < pieces;) {
-      const size_t off = k * BOUNCE_PIECE, len = std::min(BOUNCE_PIECE, bytes - off);
-      if (cudaMemcpyAsync(mine, src + off, len, cudaMemcpyDeviceToHost, c->user_stream) != cudaSuccess ||
-          cudaEventRecord(c->bounce_ev[t], c->user_stream) != cudaSuccess ||
-          cudaEventSynchronize(c->bounce_ev[t]) != cudaSuccess) {
-        failed = 1;
-        break;
-      }
-      std::memcpy(dst + off, mine, len);
-    }
-  };
-  std::vector<std::thread> th;
-  try {
-    th.reserve(n);
-    for (int t = 1; t < n; ++t) th.emplace_back(work, t);
-  } catch (...) {  // fewer threads take all the pieces
-  }
-  work(0);
-  for (auto &x : th) x.join();
-  return failed ? J2K_ERR_CUDA : J2K_OK;
+  const bool ok = j2k::copy_in_pieces(bytes, [&](int t, size_t off, size_t len) {
+    uint8_t *mine = c->h_bounce + (size_t)t * j2k::COPY_PIECE;
+    if (cudaSetDevice(c->device) != cudaSuccess ||
+        cudaMemcpyAsync(mine, src + off, len, cudaMemcpyDeviceToHost, c->user_stream) != cudaSuccess ||
+        cudaEventRecord(c->bounce_ev[t], c->user_stream) != cudaSuccess ||
+        cudaEventSynchronize(c->bounce_ev[t]) != cudaSuccess)
+      return false;
+    std::memcpy(dst + off, mine, len);
+    return true;
+  });
+  return ok ? J2K_OK : J2K_ERR_CUDA;
 }
 }  // namespace
 
@@ -1156,7 +1133,7 @@ extern "C" int j2k_gpu_output_copy(j2k_gpu_ctx *c, int slot, void *dst, size_t b
   if (bytes < im.out_bytes) return J2K_ERR_ARG;
   cudaSetDevice(c->device);
   const uint8_t *src = (const uint8_t *)c->d_out.p + im.out_base;
-  if (im.out_bytes >= BOUNCE_FROM) {
+  if (im.out_bytes >= j2k::COPY_THREADED_FROM) {
     cudaPointerAttributes at{};
     const cudaError_t e = cudaPointerGetAttributes(&at, dst);
     if (e != cudaSuccess) cudaGetLastError();

@@ -16,6 +16,7 @@
 // another; the engine starts a batch whose Tier-1 fills the GPU only after the previous
 // decode, see j2k_gpu_batch_run).
 #include "../../include/j2k_server.h"
+#include "host_copy.h"
 #include "pinned_arena.h"
 
 #include <cuda_runtime.h>
@@ -400,7 +401,14 @@ extern "C" int j2k_server_wait(j2k_server *s, int64_t id, void *dst, size_t cap,
     const uint8_t *src = r->out;
     const size_t n = r->out_bytes;
     lk.unlock();
-    std::memcpy(dst, src, n);
+    if (n < j2k::COPY_THREADED_FROM) {
+      std::memcpy(dst, src, n);
+    } else {
+      j2k::copy_in_pieces(n, [&](int, size_t off, size_t len) {
+        std::memcpy((uint8_t *)dst + off, src + off, len);
+        return true;
+      });
+    }
   }
   return J2K_OK;
 }

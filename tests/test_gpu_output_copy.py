@@ -33,3 +33,20 @@ def test_pageable_copy_equals_pinned(pkg, w, h):
         assert np.array_equal(odd[1:], want)
     finally:
         ctx.close()
+
+
+def test_service_copy_equals_view(pkg):
+    """The service's copy of a result above that size equals its page-locked original."""
+    from jpeg2000_decoder_b200 import native, synth
+    img = np.tile(synth.fields_and_edges(6, 256, 256), (1, 10, 10))[:, :2341, :2389]
+    cs = native.encode(np.ascontiguousarray(img), 8, reversible=0, levels=3, num_layers=1, layer_bpp=[0.3], tile_w=1024,
+                       tile_h=1024, guard_bits=1)
+    srv = native.Server(0)
+    try:
+        rid = srv.submit(cs, native.FMT_24BITS_RGB)
+        got = srv.result(rid)
+        rc, view = srv.view(rid)
+        assert rc == 0 and got.size == 2341 * 2389 * 3 and np.array_equal(got, view)
+        srv.release(rid)
+    finally:
+        srv.close()
