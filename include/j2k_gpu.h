@@ -155,7 +155,8 @@ typedef struct j2k_gpu_tuning {
                             the measured workloads, never chosen by the auto form; switching to or
                             from 3 takes effect at the next stage) */
   int t1_latency_waves;  /* auto form without an autotuned choice: latency form while code-blocks <=
-                            this many x 32 warps x SMs, compact above */
+                            this many x 32 warps x SMs, or while the longest code-block's serial
+                            decode dominates the queue; compact above */
   int dwt_coarse;        /* the coarse levels of each tile-component (resolutions up to 64 samples a
                             side) in one shared-memory kernel: 0 default (off), 1 on, 2 off (one
                             launch per level) */

@@ -200,6 +200,8 @@ struct j2k_gpu_ctx {
     size_t o_ctk = 0, n_ctasks[2] = {0, 0};  // coarse-level tasks: [0] 9/7, [1] 5/3
     int fwin = 1;
     int maxL = 0;
+    uint64_t coded = 0;                   // coded bytes of all blocks
+    uint32_t longest = 0, longest_passes = 0;  // of the block with most coded bytes
     std::vector<uint32_t> dtask_off;
   } sg;
   cudaEvent_t ev[6] = {};  // h2d start, h2d end, Tier-1 end, DWT end, decode end, output copies end
@@ -469,8 +471,13 @@ void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, c
 // warp form, 3 one block per lane, and warps per CTA of a warp form.  An explicit
 // tuning.t1_form wins; the auto form (0) takes the autotuned choice of the queue's size
 // bucket, else the latency form while the queue holds at most `t1_latency_waves` blocks
-// per resident warp slot of the GPU (the launch's time is then the serial time of its
-// longest blocks) and the compact form for longer queues.  The lane form is only taken
+// per resident warp slot of the GPU, and for longer queues while the serial chain of the
+// longest block still dominates: the compact form takes twice as long for it, and that is
+// paid back only once the whole queue takes about 2.2 times as long as the chain.  Measured Tier-1
+// ms, latency / compact form: 4096x2160 12-bit 9/7 pictures x2 3.95 / 7.27, x4 6.25 / 8.22, x6
+// 9.27 / 9.98; 2048x2048 9/7 x8 4.43 / 8.05; 1080p 9/7 frames x8 3.90 / 4.01, x10 4.82 / 4.50,
+// x24 11.46 / 9.58; 1080p lossless x6 12.54 / 12.29.  (Chain: 0.73 us a coded byte and 34 us a
+// pass; the compact form takes 1.3 MB of coded bytes a ms.)  The lane form is only taken
 // when asked for: on B200 it measured 4.2x slower than the compact form on 1080p 9/7
 // frames (its lanes' pass walks diverge: 4.4 of 32 threads active per instruction).
 void t1_shape(const j2k_gpu_ctx *c, int n, int &form, int &warps) {
@@ -486,7 +493,8 @@ void t1_shape(const j2k_gpu_ctx *c, int n, int &form, int &warps) {
     return;
   }
   const int waves = c->tuning.t1_latency_waves > 0 ? c->tuning.t1_latency_waves : 2;
-  form = (long long)n <= (long long)waves * c->sm_count * 32 ? 2 : 1;
+  const double chain_us = 0.73 * c->sg.longest + 34.0 * c->sg.longest_passes, queue_us = c->sg.coded / 1300.0;
+  form = (long long)n <= (long long)waves * c->sm_count * 32 || queue_us < 2.2 * chain_us ? 2 : 1;
 }
 
 // Enqueue the Tier-1 stage: the lane kernel on the lane queue and a warp form on the rest,
@@ -540,8 +548,8 @@ extern "C" int j2k_gpu_batch_stage(j2k_gpu_ctx *c, void *user_stream) {
   const bool coarse_on = c->tuning.dwt_coarse == 1 || (c->tuning.dwt_coarse == 0 && c->dwt_auto == 1);
   const bool lane_split = c->tuning.t1_form == 3;  // queue classes for the lane form
   int fwin = 1;
-  uint64_t byte_base = 0;
-  uint32_t seg_base = 0;
+  uint64_t byte_base = 0, coded = 0;
+  uint32_t seg_base = 0, longest = 0, longest_passes = 0;
   int maxL = 0;
   for (auto &im : c->imgs)
     for (auto &tc : im.plan->p.tilecomps) maxL = std::max(maxL, tc.levels);
@@ -556,6 +564,11 @@ extern "C" int j2k_gpu_batch_stage(j2k_gpu_ctx *c, void *user_stream) {
       cb.out_off += im.coef_base;
       uint32_t idx = (uint32_t)cbs.size();
       cbs.push_back(cb);
+      coded += cb.data_len;
+      if (cb.data_len > longest) {
+        longest = cb.data_len;
+        longest_passes = cb.num_passes;
+      }
       ordq[lane_split && j2k_lanes::lane_eligible(cb) ? QL : QW].push_back(idx);
     }
     seg.insert(seg.end(), p.seglens.begin(), p.seglens.end());
@@ -834,6 +847,9 @@ extern "C" int j2k_gpu_batch_stage(j2k_gpu_ctx *c, void *user_stream) {
   CK(cudaEventRecord(c->ev[1], st));
   for (int q = 0; q < NQ; ++q) c->sg.nq[q] = ordq[q].size();
   c->sg.n_cblks = S.cblks;
+  c->sg.coded = coded;
+  c->sg.longest = longest;
+  c->sg.longest_passes = longest_passes;
   c->sg.n_otasks = otasks.size();
   c->sg.o_fgr = o_fgr;
   c->sg.o_ftk = o_ftk;
