@@ -112,14 +112,32 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
       __threadfence();
       __syncwarp();
       const bool irrev = (cb.flags & J2K_CB_IRREV) != 0;
-      for (int y = 0; y < h; ++y) {
-        int32_t *r = blk + (size_t)y * cb.out_stride;
-        const uint32_t sig = 1u << (SIG_POS + 3 * (y & 3));
-        const uint32_t *wrow = b.cw + (y >> 2) * b.gap;
-        for (int x = lane; x < w; x += 32) {
-          const int32_t v = (wrow[x] & sig) ? __ldcg(r + x) : 0;
-          if (irrev) *reinterpret_cast<float *>(r + x) = __fmul_rn((float)signmag_to_int(v), cb.gain);
-          else r[x] = place53(v, cb.mb);
+      // a stripe column's four samples at a time: one context word, four loads under way (eight in
+      // the latency form; the throughput form has no registers for them).  Against a row at a
+      // time, one load under way: 2048x2048 RGB 9/7 3.44 -> 3.23 ms, 512x512 gray 2.76 -> 2.59.
+      auto column = [&](int s, int x) {
+        const uint32_t word = b.cw[s * b.gap + x];
+        int32_t *r = blk + (size_t)(4 * s) * cb.out_stride + x;
+        const int rows = min(4, h - 4 * s);
+        int32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          v[k] = k < rows && (word >> (SIG_POS + 3 * k)) & 1 ? __ldcg(r + (size_t)k * cb.out_stride) : 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k >= rows) continue;
+          int32_t *o = r + (size_t)k * cb.out_stride;
+          if (irrev) *reinterpret_cast<float *>(o) = __fmul_rn((float)signmag_to_int(v[k]), cb.gain);
+          else *o = place53(v[k], cb.mb);
+        }
+      };
+      for (int x = lane; x < w; x += 32) {
+        if constexpr (LATENCY) {
+#pragma unroll 2
+          for (int s = 0; s < b.stripes; ++s) column(s, x);
+        } else {
+#pragma unroll 1
+          for (int s = 0; s < b.stripes; ++s) column(s, x);
         }
       }
     }
@@ -130,9 +148,10 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
 
 // The two kernel forms.  The throughput (compact) form keeps the default register target,
 // which leaves room for 32 resident warps per SM; the latency form (batches that fit about two
-// waves) may use more registers, as occupancy does not bound it, and has one warp a CTA: its
-// shared-memory addresses are constants then (one 2048x2048 RGB 9/7 picture 3.86 -> 3.63 ms, one
-// 256x256 picture 1.14 -> 1.04 ms against CTAs of eight warps).
+// waves) may use more registers, as occupancy does not bound it (17 warps per SM at 117; at 76
+// to 90 it takes 3 to 8 % longer), and has one warp a CTA: its shared-memory addresses are
+// constants then (one 2048x2048 RGB 9/7 picture 3.86 -> 3.63 ms, one 256x256 picture 1.14 ->
+// 1.04 ms against CTAs of eight warps).
 #define J2K_T1_PARAMS                                                                                   \
   const j2k_cblk *__restrict__ cbs, const uint32_t *__restrict__ order, int n, int *__restrict__ counter, \
       const uint8_t *__restrict__ bytes, const uint32_t *__restrict__ seglens, void *__restrict__ coef,   \
@@ -142,7 +161,7 @@ __global__ void __launch_bounds__(256) t1_kernel_compact(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, false>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 template <int MAXW, int MAXH>
-__global__ void __launch_bounds__(32, 16) t1_kernel_latency(J2K_T1_PARAMS) {
+__global__ void __launch_bounds__(32, 12) t1_kernel_latency(J2K_T1_PARAMS) {
   t1_body<MAXW, MAXH, true>(cbs, order, n, counter, bytes, seglens, coef, status);
 }
 #undef J2K_T1_PARAMS
