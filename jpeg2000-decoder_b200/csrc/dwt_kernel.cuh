@@ -9,14 +9,13 @@
  * lifting eight outputs at a time in registers, and stores the 64x64 result from the column
  * pass.  Every level is one read and one write of the level's samples; all tile-components
  * of a batch at a given level share one launch.
- * The kernels are bound by instruction issue (74 % of the slots in the 4096x2160 level, DRAM
- * 1.0 TB/s) and, in small levels, by the latency of one tile, so the work is cut into short
- * independent chains and the staging walks lines with pointers.  Measured on B200 against a
- * thread per 72-sample line streamed through shared memory: a 4096x2160 9/7 plane of five
- * levels 75.4 -> 45.7 us, a 1000x777 5/3 tile 43.8 -> 21.8 us (one cooperative launch with
- * 32x32 tiles in the small levels; five launches of these kernels 61.6 and 32.8 us), the
- * DWT + MCT stage of 32 1080p frames 0.955 -> 0.81 ms.  Five resident CTAs at 48 registers
- * instead of four at 64 took 51.2 us (spills).
+ * The kernels are bound by instruction issue and the latency of a tile's phases (59 % of the
+ * issue slots in the 4096x2160 level, DRAM 1.3 TB/s), so the work is cut into short independent
+ * chains, the staging walks lines with pointers, and a tile's copies run under the column pass
+ * of the tile before it.  Measured on B200 against a thread per 72-sample line streamed through
+ * shared memory: a 4096x2160 9/7 plane of five levels 75.4 -> 43.3 us, a 1000x777 5/3 tile
+ * 43.8 -> 18.5 us (one cooperative launch with 32x32 tiles in the small levels), the DWT + MCT
+ * stage of 32 1080p frames 0.955 -> 0.79 ms.
  *
  * Arithmetic follows the reference exactly so that results are bit-identical:
  *   9/7: each lifting update is D = S - c * (L + R) with three separately rounded float
@@ -227,22 +226,24 @@ __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const W
         copy(base + (size_t)(mirror(oy - DWT_H + warp + WARPS * i, rh) >> 1) * stride, d0 + 4 * PITCH * WARPS * i);
     }
   }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
 }
 
 // Rebuild the TILE x TILE output tile at (ox, oy) of one level for `nw` windows of the same
 // geometry (the components of one tile at their last level, or one tile-component).  The
 // results are left in the centre of each window, S[w].tile[(y + 4) * PITCH + x + 4], or
-// (DIRECT: a single window, its rows in `mid`) stored to `out` from the column pass.
-template <bool REV, bool DIRECT, int TILE>
+// (DIRECT: a single window, its rows in `mid`) stored to `out` from the column pass.  `staged`: the
+// window is already on its way; `window_free` is called once the window has been read for the
+// last time (DIRECT: the next tile's copies then run under the column pass).
+template <bool REV, bool DIRECT, int TILE, class F>
 __device__ __forceinline__ void dwt_windows(DwtSmem<REV, TILE> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
                                             int lh, bool ll_gain, float gain, bool refcompat, int ox, int oy,
                                             typename DwtTypes<REV>::T *mid, typename DwtTypes<REV>::T *out,
-                                            int stride_out) {
+                                            int stride_out, bool staged, F window_free) {
   typedef typename DwtTypes<REV>::T T;
   constexpr int N = DwtSmem<REV, TILE>::N, PITCH = DwtSmem<REV, TILE>::PITCH, MID_PITCH = TILE + 1;
-  dwt_stage<REV, TILE>(S, nw, src, rw, rh, lw, lh, ox, oy);
+  if (!staged) dwt_stage<REV, TILE>(S, nw, src, rw, rh, lw, lh, ox, oy);
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
   // Rows: a thread lifts eight outputs of a row; consecutive threads take consecutive rows (the
   // odd pitch keeps the banks apart).  The reconstructed LL entering a finer 9/7 level is
   // scaled by K_lo^2 on the way.
@@ -333,6 +334,7 @@ __device__ __forceinline__ void dwt_windows(DwtSmem<REV, TILE> *S, int nw, const
   };
   const int c = threadIdx.x % TILE;
   if (DIRECT) {
+    if (!fix) window_free();
 #pragma unroll 1
     for (int seg = threadIdx.x / TILE; seg < SEGS; seg += STEP) {
       T y[SEG];
@@ -395,18 +397,39 @@ __device__ __forceinline__ void dwt_windows(DwtSmem<REV, TILE> *S, int nw, const
       if (yy < oh && xx < ow)
         out[(size_t)(oy + yy) * stride_out + ox + xx] = S[0].tile[(yy + DWT_H) * PITCH + xx + DWT_H];
     }
+    __syncthreads();
+    window_free();
   }
 }
 
-// One output tile of one level of one tile-component, stored to `out`.
-template <bool REV, int TILE>
-__device__ __forceinline__ void dwt_tile(LevelSmem<REV, TILE> &S, const typename DwtTypes<REV>::T *quad, int stride_q,
-                                         const typename DwtTypes<REV>::T *llsrc, int stride_ll,
-                                         typename DwtTypes<REV>::T *out, int stride_out, int rw, int rh, int lw,
-                                         int lh, bool ll_gain, float gain, bool refcompat, int ox, int oy) {
-  const WinSrc<REV> src{quad, stride_q, llsrc, stride_ll};
-  dwt_windows<REV, true, TILE>(&S.win, 1, &src, rw, rh, lw, lh, ll_gain, gain, refcompat, ox, oy, S.mid, out, stride_out);
-  __syncthreads();  // the window is free for the next tile
+// One level of one tile-component, as a tile's kernel needs it
+template <bool REV>
+struct LevelArgs {
+  WinSrc<REV> src;
+  typename DwtTypes<REV>::T *out;
+  int stride_out, rw, rh, lw, lh, ox, oy;  // (ox, oy): the tile
+  bool ll_gain, refcompat;
+};
+// Output tiles of levels, stored to their `out`, one after the other: next(args) sets the next
+// tile's arguments or returns false.  The copies of a tile's window run under the column pass of
+// the tile before it.
+template <bool REV, int TILE, class Next>
+__device__ __forceinline__ void dwt_tiles(LevelSmem<REV, TILE> &S, float gain, Next next) {
+  LevelArgs<REV> cur, ahead;
+  bool more = next(cur);
+  if (more) dwt_stage<REV, TILE>(&S.win, 1, &cur.src, cur.rw, cur.rh, cur.lw, cur.lh, cur.ox, cur.oy);
+  while (more) {
+    bool then = false;
+    dwt_windows<REV, true, TILE>(&S.win, 1, &cur.src, cur.rw, cur.rh, cur.lw, cur.lh, cur.ll_gain, gain, cur.refcompat,
+                                 cur.ox, cur.oy, S.mid, cur.out, cur.stride_out, true, [&] {
+                                   then = next(ahead);
+                                   if (then)
+                                     dwt_stage<REV, TILE>(&S.win, 1, &ahead.src, ahead.rw, ahead.rh, ahead.lw, ahead.lh,
+                                                          ahead.ox, ahead.oy);
+                                 });
+    cur = ahead;
+    more = then;
+  }
 }
 
 template <bool REV>
@@ -415,15 +438,25 @@ __global__ void __launch_bounds__(DWT_THREADS) dwt_level_kernel(const DwtLevel *
                                                         void *bufB, void *bufC, float ll_gain_value) {
   typedef typename DwtTypes<REV>::T T;
   __shared__ LevelSmem<REV> S;
-  for (int task = blockIdx.x; task < ntasks; task += gridDim.x) {
+  int task = blockIdx.x;
+  dwt_tiles<REV, DWT_T>(S, ll_gain_value, [&](LevelArgs<REV> &a) {
+    if (task >= ntasks) return false;
     const DwtTask tk = tasks[task];
     const DwtLevel L = levels[tk.level];
-    const T *A = dwt_buf<REV>(0, bufA, bufB, bufC) + L.base;
-    const T *LLsrc = dwt_buf<REV>(L.ll_src, bufA, bufB, bufC) + L.base;
-    T *out = dwt_buf<REV>(L.out_dst, bufA, bufB, bufC) + L.base;
-    dwt_tile<REV, DWT_T>(S, A, L.stride, LLsrc, L.stride, out, L.stride, L.rw, L.rh, L.lw, L.lh, L.ll_gain != 0,
-                  ll_gain_value, L.refcompat != 0, tk.tx * DWT_T, tk.ty * DWT_T);
-  }
+    task += gridDim.x;
+    a.src = {dwt_buf<REV>(0, bufA, bufB, bufC) + L.base, L.stride, dwt_buf<REV>(L.ll_src, bufA, bufB, bufC) + L.base, L.stride};
+    a.out = dwt_buf<REV>(L.out_dst, bufA, bufB, bufC) + L.base;
+    a.stride_out = L.stride;
+    a.rw = L.rw;
+    a.rh = L.rh;
+    a.lw = L.lw;
+    a.lh = L.lh;
+    a.ox = tk.tx * DWT_T;
+    a.oy = tk.ty * DWT_T;
+    a.ll_gain = L.ll_gain != 0;
+    a.refcompat = L.refcompat != 0;
+    return true;
+  });
 }
 
 // ------------------------------------------------------------------ output stage -------
@@ -598,7 +631,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 3) last_level_output_kernel(con
     }
     const int ox = tk.tx * DWT_T, oy = tk.ty * DWT_T;
     dwt_windows<REV, false, DWT_T>(S, nc, src, F.rw, F.rh, F.lw, F.lh, F.ll_gain != 0, ll_gain_value, F.refcompat != 0, ox, oy,
-                            nullptr, nullptr, 0);
+                            nullptr, nullptr, 0, false, [] {});
     const int ow = min(DWT_T, F.rw - ox), oh = min(DWT_T, F.rh - oy);
     if (G.fmt == 2 && G.bitdepth == 8 && G.mct && nc == 3) {
       // 24-bit RGB after the inverse MCT (the common path): sixteen pixels per thread (48
@@ -795,9 +828,12 @@ struct AllLevels {
 };
 // A level that 64x64 tiles would spread over less than half of the CTAs is cut into 32x32 tiles:
 // more of the chip works on it, each CTA for a shorter time.
+// Two CTAs an SM: with the next window's copies under way they take a 4096x2160 plane as fast as
+// four (43.3 us against 46.5), and the barriers between the levels are cheaper (a 1000x777 tile
+// 18.5 us against 20.6).
 constexpr int SMALL_T = 32;
 template <bool REV>
-__global__ void __launch_bounds__(DWT_THREADS) dwt_all_levels_kernel(const AllLevels<REV> L) {
+__global__ void __launch_bounds__(DWT_THREADS, 2) dwt_all_levels_kernel(const AllLevels<REV> L) {
   typedef typename DwtTypes<REV>::T T;
   __shared__ __align__(16) uint8_t smem[sizeof(LevelSmem<REV, DWT_T>)];
   for (int r = 1; r <= L.levels; ++r) {
@@ -809,9 +845,14 @@ __global__ void __launch_bounds__(DWT_THREADS) dwt_all_levels_kernel(const AllLe
     auto level = [&](auto edge) {
       constexpr int E = decltype(edge)::value;
       const int tiles_x = (rw + E - 1) / E, tiles = tiles_x * ((rh + E - 1) / E);
-      for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-        dwt_tile<REV, E>(*reinterpret_cast<LevelSmem<REV, E> *>(smem), L.coef, L.coef_stride, ll, ll_stride, dst, dst_stride,
-                         rw, rh, lw, lh, !REV && r > 1, L.ll_gain, L.refcompat != 0, (t % tiles_x) * E, (t / tiles_x) * E);
+      int t = blockIdx.x;
+      dwt_tiles<REV, E>(*reinterpret_cast<LevelSmem<REV, E> *>(smem), L.ll_gain, [&](LevelArgs<REV> &a) {
+        if (t >= tiles) return false;
+        a = {{L.coef, L.coef_stride, ll, ll_stride}, dst, dst_stride, rw, rh, lw, lh, (t % tiles_x) * E, (t / tiles_x) * E,
+             !REV && r > 1, L.refcompat != 0};
+        t += gridDim.x;
+        return true;
+      });
     };
     const int large = ((rw + DWT_T - 1) / DWT_T) * ((rh + DWT_T - 1) / DWT_T);
     if (2 * large <= (int)gridDim.x) level(std::integral_constant<int, SMALL_T>{});

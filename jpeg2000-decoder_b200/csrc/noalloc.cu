@@ -80,8 +80,9 @@ int resident_ctas() {
           cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;
-  known[dev].store(n * sms, std::memory_order_relaxed);
-  return n * sms;
+  n = std::min(n, 2) * sms;  // as many as the kernel is laid out for
+  known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 template <bool REV>
