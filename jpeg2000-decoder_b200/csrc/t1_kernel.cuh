@@ -482,7 +482,7 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
       uint32_t *mine = out + c0 + lane;
       uint32_t live = __ballot_sync(0xffffffffu, valid && pass_rows<PASS>(word));
       uint32_t zero = PASS == P_CLEANUP ? __ballot_sync(0xffffffffu, valid && word == 0) : 0u;
-      const uint32_t inside = b.w - c0 >= 32 ? 0xffffffffu : (1u << (b.w - c0)) - 1u;
+      const uint32_t inside = __ballot_sync(0xffffffffu, valid);
       while (live) {
         const int bit = __ffs(live) - 1;
         uint32_t *wp = row + c0 + bit;
@@ -543,9 +543,9 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
             if (RAW) {
               d = raw_bit(raw);
             } else {
+              mq_ready<LATENCY>(mq);
               const uint32_t off = b.zc[(W >> k3) & 0x1EF];
               uint2 e = *reinterpret_cast<const uint2 *>(b.cx + off);
-              mq_ready<LATENCY>(mq);
               d = mq_symbol<LATENCY>(mq, b.cx + off, e, b.mq);
             }
             if (!is_one(d)) continue;
@@ -564,9 +564,6 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
           sign &= 1u << 31;
           hit = 0xffffffffu;
           W |= ((1u << SIG_POS) | (sign >> (31 - CHI_POS))) << k3;
-          __syncwarp();
-          spread(b, wp, k3, sign);
-          __syncwarp();
           // (the latency form keeps its lane's column address, the throughput form the registers)
           put_sample((LATENCY ? mine : out + c0 + bit) + (k3 * 11 >> 5) * b.stride, sign + (3u << p >> 1),
                      lane == bit);
@@ -574,6 +571,9 @@ __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq,
             x = pass_rows<PASS>(W) & (0xFFFFFFF8u << k3);
             W |= x << PI_POS;
           }
+          __syncwarp();
+          spread(b, wp, k3, sign);
+          __syncwarp();
         }
         *wp = W;
         const uint32_t right = (2u << bit) & inside & hit;
