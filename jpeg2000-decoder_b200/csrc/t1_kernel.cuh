@@ -35,9 +35,9 @@
  * without renormalisation (fewest instructions), the latency form has no branch in a symbol and
  * takes refinement symbols four at a time (shortest chain).
  * Measured against the form with a renormalisation loop, a byte at a time, rows unrolled
- * (B200, Tier-1 ms): one 2048x2048 RGB 9/7 picture 7.22 -> 3.83, one 512x512 gray lossless
- * picture 4.92 -> 3.2, one 2048x1080 12-bit BYPASS + RESET picture 5.47 -> 3.16, 32 1080p 9/7
- * frames 14.76 -> 13.2.
+ * (B200, Tier-1 ms): one 2048x2048 RGB 9/7 picture 7.22 -> 3.2, one 512x512 gray lossless
+ * picture 4.92 -> 2.54, one 256x256 RGB 9/7 picture 1.62 -> 0.90, one 2048x1080 12-bit BYPASS +
+ * RESET picture 5.47 -> 2.83, 32 1080p 9/7 frames 14.76 -> 12.54.
  *
  * Semantics follow the reference block decoder exactly (decoder/codec/src/
  * bmi_block_decoder.cpp:10-853, bmi_mq_decoder.h/.cpp, bmi_t1_macro.h): same context-word

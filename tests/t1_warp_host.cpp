@@ -117,7 +117,7 @@ extern "C" int t1_warp_host_block(const j2k_cblk *cb, const uint8_t *bytes, cons
     ready = true;
   }
   typedef T1Layout<64, 64> Lay;
-  // exactly the device's area, filled with garbage; sized blocks so a checker sees an overrun
+  // exactly the device's area, filled with garbage, in allocations of their own size
   uint8_t *mem = (uint8_t *)aligned_alloc(16, Lay::PER_WARP);
   std::memset(mem, 0xA5, Lay::PER_WARP);
   uint8_t *slots = (uint8_t *)aligned_alloc(16, (size_t)LANES * (Lay::BITS - Lay::CX));
