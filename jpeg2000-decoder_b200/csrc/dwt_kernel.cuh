@@ -30,7 +30,9 @@
  * reference's per-step mirroring at the region edges.
  */
 #pragma once
+#ifdef __CUDACC__
 #include <cooperative_groups.h>
+#endif
 
 #include <cstdint>
 #include <type_traits>
@@ -86,13 +88,21 @@ struct OutTask {
 };
 
 // Source position of window position p on a line of n samples: whole-sample symmetric
-// extension, which keeps the parity.  Positions more than four past the end feed no output:
-// they are brought back to one that exists.
+// extension, which keeps the parity on lines of two and more samples.  Positions more than four
+// past the end feed no output: they are brought back to one that exists.
 __device__ __forceinline__ int mirror(int p, int n) {
   if (n == 1) return 0;
   if (p > n + 3) p = n + 3 - ((n + 3 - p) & 1);
   while (p < 0 || p >= n) p = p < 0 ? -p : 2 * (n - 1) - p;
   return p;
+}
+
+// Where that sample lies on the de-interleaved line, whose low part has lo samples.  The part
+// follows from the mirrored position: the only sample of a line of one is its low part, whatever
+// the parity of p.
+__device__ __forceinline__ int window_source(int p, int n, int lo) {
+  const int x = mirror(p, n);
+  return ((x & 1) ? lo : 0) + (x >> 1);
 }
 
 __device__ __forceinline__ float lift97(float s, float c, float l, float r) {
@@ -184,12 +194,24 @@ struct WinSrc {
   int stride_ll;
 };
 
+// One asynchronous copy of the staging, `to` a shared-memory address
+template <typename T>
+__device__ __forceinline__ void stage_copy(uint32_t to, const T *from) {
+#ifdef __CUDACC__
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(to), "l"(from));
+#else
+  host_stage_copy(to, from);  // of the including file
+#endif
+}
+
 // Stage the window of the tile at (ox, oy) with asynchronous 4-byte copies: every thread issues
 // all of its loads before waiting.  A warp copies a window row: lane l holds positions l,
 // l + 32 and l + 64 (as far as the row goes), even ones from the low part and odd ones from the
-// high part of the line (64 contiguous bytes of each per copy).  The mirror keeps the parity
-// and the warps' number is even, so a lane's part and a warp's row part never change: inside the
-// level a warp's pointers advance by whole lines.
+// high part of the line (64 contiguous bytes of each per copy).  The warps' number is even, so the
+// parity of a lane's columns and of a warp's rows never changes: a lane and warp of even parity
+// take LL, the others the level's quadrants (a line of one sample has only its low part, which
+// odd positions then read as well; no output comes from them), and inside the level a warp's
+// pointers advance by whole lines.
 template <bool REV, int TILE>
 __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
                                           int lh, int ox, int oy) {
@@ -201,29 +223,28 @@ __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const W
   const int odd = lane & 1, high = warp & 1;
   int col[COLS];
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) col[j] = (mirror(ox - DWT_H + lane + 32 * j, rw) >> 1) + (odd ? lw : 0);
+  for (int j = 0; j < COLS; ++j) col[j] = window_source(ox - DWT_H + lane + 32 * j, rw, lw);
   const bool last = lane < N - 32 * (COLS - 1);
   const bool inside = oy >= DWT_H && oy + TILE + DWT_H <= rh;
   for (int w = 0; w < nw; ++w) {
     const bool ll = !high && !odd;
-    const T *base = ll ? src[w].llsrc : src[w].quad + (high ? (size_t)lh * src[w].stride_q : 0);
+    const T *base = ll ? src[w].llsrc : src[w].quad;
     const int stride = ll ? src[w].stride_ll : src[w].stride_q;
     const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(S[w].tile + warp * PITCH + lane);
     auto copy = [&](const T *line, uint32_t d) {
 #pragma unroll
       for (int j = 0; j < COLS; ++j)
-        if (j < COLS - 1 || last)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d + 128 * j), "l"(line + col[j]));
+        if (j < COLS - 1 || last) stage_copy(d + 128 * j, line + col[j]);
     };
     if (inside) {
-      const T *line = base + (size_t)((oy - DWT_H + warp) >> 1) * stride;
+      const T *line = base + (size_t)window_source(oy - DWT_H + warp, rh, lh) * stride;
       const size_t step = (size_t)(WARPS / 2) * stride;
 #pragma unroll
       for (int i = 0; i < N / WARPS; ++i, line += step) copy(line, d0 + 4 * PITCH * WARPS * i);
     } else {
 #pragma unroll 1
       for (int i = 0; i < N / WARPS; ++i)
-        copy(base + (size_t)(mirror(oy - DWT_H + warp + WARPS * i, rh) >> 1) * stride, d0 + 4 * PITCH * WARPS * i);
+        copy(base + (size_t)window_source(oy - DWT_H + warp + WARPS * i, rh, lh) * stride, d0 + 4 * PITCH * WARPS * i);
     }
   }
 }
