@@ -189,7 +189,8 @@ int j2k_gpu_autotune(j2k_gpu_ctx *ctx, void *stream, int iters, j2k_gpu_tuning *
  * again.  Overlapping calls race on the array.  A resolution table that does not nest
  * inside the tile-component returns J2K_ERR_ARG before anything is enqueued; a CUDA error
  * already pending from earlier work returns J2K_ERR_CUDA and stays pending.
- * Asynchronous on `stream`. */
+ * Asynchronous on `stream`, which may be one that is being captured or one whose work may use
+ * only some of the SMs; no level needs the whole device free. */
 #define J2K_NOALLOC_SCRATCH_BYTES ((size_t)32 << 20)
 int j2k_gpu_tile_idwt_noalloc(const j2k_tilecomp *tc, int reversible, int flags, const void *coef, void *out,
                               int out_stride, void *stream);

@@ -14,8 +14,8 @@
  * chains, the staging walks lines with pointers, and a tile's copies run under the column pass
  * of the tile before it.  Measured on B200 against a thread per 72-sample line streamed through
  * shared memory: a 4096x2160 9/7 plane of five levels 75.4 -> 43.3 us, a 1000x777 5/3 tile
- * 43.8 -> 18.5 us (one cooperative launch with 32x32 tiles in the small levels), the DWT + MCT
- * stage of 32 1080p frames 0.955 -> 0.79 ms.
+ * 43.8 -> 16.6 us (a programmatic launch per level, 32x32 tiles in the small levels), the DWT +
+ * MCT stage of 32 1080p frames 0.955 -> 0.79 ms.
  *
  * Arithmetic follows the reference exactly so that results are bit-identical:
  *   9/7: each lifting update is D = S - c * (L + R) with three separately rounded float
@@ -30,10 +30,6 @@
  * reference's per-step mirroring at the region edges.
  */
 #pragma once
-#ifdef __CUDACC__
-#include <cooperative_groups.h>
-#endif
-
 #include <cstdint>
 #include <type_traits>
 
@@ -833,53 +829,43 @@ __global__ void __launch_bounds__(128) dwt_coarse_kernel(const CoarseTask *__res
 
 namespace j2k_dev {
 
-// Every level of one tile-component in one cooperative launch, all buffers given explicitly (no
-// descriptor tables in device memory); CTAs take the 64x64 output tiles of a level in turn and
-// meet at a grid-wide barrier between levels.  Used by the entry point that runs on a static
-// scratch array (noalloc.cu), whose levels are mostly small: a launch each cost 5 to 6 us.
+// One level of one tile-component, all buffers given explicitly (no descriptor tables in device
+// memory).  Used by the entry point that runs on a static scratch array (noalloc.cu).
 template <bool REV>
-struct AllLevels {
+struct OneLevel {
   typedef typename DwtTypes<REV>::T T;
-  const T *coef;  // Mallat layout, row stride coef_stride
-  T *half[2];     // intermediate resolutions (level r to half[r & 1]), row stride half_stride
+  const T *coef, *ll;  // Mallat layout (row stride coef_stride) and the LL quadrant (ll_stride)
   T *out;
-  int coef_stride, half_stride, out_stride, levels, refcompat;
+  int coef_stride, ll_stride, out_stride, rw, rh, lw, lh;
+  int scale_ll, refcompat, more;  // more: another level follows
   float ll_gain;
-  int res_w[J2K_MAX_LEVELS + 1], res_h[J2K_MAX_LEVELS + 1];
 };
-// A level that 64x64 tiles would spread over less than half of the CTAs is cut into 32x32 tiles:
-// more of the chip works on it, each CTA for a shorter time.
-// Two CTAs an SM: with the next window's copies under way they take a 4096x2160 plane as fast as
-// four (43.3 us against 46.5), and the barriers between the levels are cheaper (a 1000x777 tile
-// 18.5 us against 20.6).
-constexpr int SMALL_T = 32;
-template <bool REV>
-__global__ void __launch_bounds__(DWT_THREADS, 2) dwt_all_levels_kernel(const AllLevels<REV> L) {
-  typedef typename DwtTypes<REV>::T T;
-  __shared__ __align__(16) uint8_t smem[sizeof(LevelSmem<REV, DWT_T>)];
-  for (int r = 1; r <= L.levels; ++r) {
-    const int rw = L.res_w[r], rh = L.res_h[r], lw = L.res_w[r - 1], lh = L.res_h[r - 1];
-    const T *ll = r == 1 ? L.coef : L.half[(r - 1) & 1];
-    const int ll_stride = r == 1 ? L.coef_stride : L.half_stride;
-    T *dst = r == L.levels ? L.out : L.half[r & 1];
-    const int dst_stride = r == L.levels ? L.out_stride : L.half_stride;
-    auto level = [&](auto edge) {
-      constexpr int E = decltype(edge)::value;
-      const int tiles_x = (rw + E - 1) / E, tiles = tiles_x * ((rh + E - 1) / E);
-      int t = blockIdx.x;
-      dwt_tiles<REV, E>(*reinterpret_cast<LevelSmem<REV, E> *>(smem), L.ll_gain, [&](LevelArgs<REV> &a) {
-        if (t >= tiles) return false;
-        a = {{L.coef, L.coef_stride, ll, ll_stride}, dst, dst_stride, rw, rh, lw, lh, (t % tiles_x) * E, (t / tiles_x) * E,
-             !REV && r > 1, L.refcompat != 0};
-        t += gridDim.x;
-        return true;
-      });
-    };
-    const int large = ((rw + DWT_T - 1) / DWT_T) * ((rh + DWT_T - 1) / DWT_T);
-    if (2 * large <= (int)gridDim.x) level(std::integral_constant<int, SMALL_T>{});
-    else level(std::integral_constant<int, DWT_T>{});
-    if (r < L.levels) cooperative_groups::this_grid().sync();
-  }
+// A level of at most two 64x64 tiles an SM is cut into 32x32 tiles: more of the chip works on it,
+// each CTA for a shorter time (the 1000x777 level, 208 large tiles: a 5/3 tile-component of that
+// size takes 16.6 us, 19.0 with large ones; 4096x2160 with 560 and 2176 tiles is left as it is).
+constexpr int SMALL_T = 32, SMALL_MOST = 2 * 148;
+// The next level's CTAs may be launched while this one drains (programmatic launch) and wait here
+// for its results, so a level costs no launch latency: 256x256, 1000x777 and 4096x2160 planes of
+// five levels take 24.8, 28.5 and 57.3 us from call to result, against 33.6, 36.3 and 64.5 with
+// plain launches and 27.4, 32.4 and 58.7 as one cooperative launch (calls one behind the other,
+// inputs not in L2, last two: 18.5 and 47.4 us, cooperative 18.7 and 46.9).  No CTA waits for one
+// that is not yet running, so the levels need no part of the GPU to themselves, as a cooperative
+// launch does: that is refused where the caller may use fewer SMs, and waits until work on other
+// streams has left every SM room.
+template <bool REV, int TILE>
+__global__ void __launch_bounds__(DWT_THREADS) dwt_one_level_kernel(const OneLevel<REV> L) {
+  __shared__ LevelSmem<REV, TILE> S;
+  if (L.more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int tiles_x = (L.rw + TILE - 1) / TILE, tiles = tiles_x * ((L.rh + TILE - 1) / TILE);
+  int t = blockIdx.x;
+  dwt_tiles<REV, TILE>(S, L.ll_gain, [&](LevelArgs<REV> &a) {
+    if (t >= tiles) return false;
+    a = {{L.coef, L.coef_stride, L.ll, L.ll_stride}, L.out, L.out_stride, L.rw, L.rh, L.lw, L.lh, (t % tiles_x) * TILE,
+         (t / tiles_x) * TILE, L.scale_ll != 0, L.refcompat != 0};
+    t += gridDim.x;
+    return true;
+  });
 }
 
 }  // namespace j2k_dev

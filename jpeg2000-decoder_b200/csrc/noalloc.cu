@@ -6,9 +6,9 @@
  * fail, and hosts that hand the library pre-allocated input and output buffers from their
  * own arena and forbid it any other device allocation.  Those callers pass the Tier-1
  * coefficients of one tile-component and an output buffer; the intermediate resolution
- * levels live in a file-scope static device array instead of pooled buffers.  All levels run in
- * one cooperative launch (a launch per level cost 5 to 6 us of host and device time each), which
- * a stream capture records like any other launch.
+ * levels live in a file-scope static device array instead of pooled buffers.  Each level is a
+ * launch that overlaps the end of the one before (programmatic launch); a stream capture records
+ * them like any other launches, and they run on whatever part of the GPU is free.
  *
  * The array is J2K_NOALLOC_SCRATCH_BYTES (32 MiB) and every GPU that loads the library
  * holds it until the process exits.  In host code the array's name is only a host-side
@@ -31,7 +31,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 
 #include "../../include/j2k_gpu.h"
@@ -69,56 +68,54 @@ int scratch_for_current_device(void **addr) {
   return J2K_OK;
 }
 
-// CTAs of the all-levels kernel that are resident on the current device together
-template <bool REV>
-int resident_ctas() {
-  static std::atomic<int> known[kMaxDevices];
-  int dev = 0, n = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-  if ((n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, j2k_dev::dwt_all_levels_kernel<REV>, j2k_dev::DWT_THREADS, 0) !=
-          cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return 0;
-  n = std::min(n, 2) * sms;  // as many as the kernel is laid out for
-  known[dev].store(n, std::memory_order_relaxed);
-  return n;
-}
+// Most CTAs of a launch (a 4096x2160 plane of 2176 tiles: 47.4 us with a CTA each, 47.8 with eight
+// CTAs an SM taking them in turn, 49.8 with five)
+constexpr int64_t kMaxCtas = 32 * 148;
 
 template <bool REV>
 int run_levels(const j2k_tilecomp &tc, int flags, const void *coef, void *out, int out_stride, cudaStream_t st,
                void *scratch) {
   typedef typename j2k_dev::DwtTypes<REV>::T T;
   const int L = tc.levels;
+  const int sw = L >= 2 ? tc.res_w[L - 1] : 1;
   const size_t half_elems = L >= 2 ? (size_t)tc.res_w[L - 1] * tc.res_h[L - 1] : 0;
-  j2k_dev::AllLevels<REV> P{};
+  T *half[2] = {reinterpret_cast<T *>(scratch), reinterpret_cast<T *>(scratch) + half_elems};
+  j2k_dev::OneLevel<REV> P{};
   P.coef = reinterpret_cast<const T *>(coef);
-  P.half[0] = reinterpret_cast<T *>(scratch);
-  P.half[1] = reinterpret_cast<T *>(scratch) + half_elems;
-  P.out = reinterpret_cast<T *>(out);
   P.coef_stride = tc.w;
-  P.half_stride = L >= 2 ? tc.res_w[L - 1] : 1;
-  P.out_stride = out_stride;
-  P.levels = L;
   P.refcompat = (flags & J2K_FLAG_REF_COMPAT) ? 1 : 0;
   P.ll_gain = j2k::irrev_ll_gain();
-  for (int r = 0; r <= L; ++r) {
-    P.res_w[r] = tc.res_w[r];
-    P.res_h[r] = tc.res_h[r];
-  }
-  // the grid: a CTA for every 32x32 tile of the finest level, as far as they are resident together
-  constexpr int E = j2k_dev::SMALL_T;
-  const int64_t tiles = (int64_t)((tc.w + E - 1) / E) * ((tc.h + E - 1) / E);
-  const int most = resident_ctas<REV>();
-  if (most <= 0) {
-    cudaGetLastError();
-    return J2K_ERR_CUDA;
-  }
-  void *args[] = {&P};
-  if (cudaLaunchCooperativeKernel((const void *)j2k_dev::dwt_all_levels_kernel<REV>, dim3((unsigned)std::min<int64_t>(tiles, most)),
-                                  dim3(j2k_dev::DWT_THREADS), args, 0, st) != cudaSuccess) {
-    cudaGetLastError();  // nothing was pending on entry: this error is ours
-    return J2K_ERR_CUDA;
+  bool first = true;
+  for (int r = 1; r <= L; ++r) {
+    P.rw = tc.res_w[r];
+    P.rh = tc.res_h[r];
+    P.lw = tc.res_w[r - 1];
+    P.lh = tc.res_h[r - 1];
+    if (P.rw <= 0 || P.rh <= 0) continue;
+    P.ll = r == 1 ? P.coef : half[(r - 1) & 1];
+    P.ll_stride = r == 1 ? tc.w : sw;
+    P.out = r == L ? reinterpret_cast<T *>(out) : half[r & 1];
+    P.out_stride = r == L ? out_stride : sw;
+    P.scale_ll = !REV && r > 1;
+    P.more = r < L;
+    auto tiles = [&](int edge) { return (int64_t)((P.rw + edge - 1) / edge) * ((P.rh + edge - 1) / edge); };
+    const bool small = tiles(j2k_dev::DWT_T) <= j2k_dev::SMALL_MOST;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min(tiles(small ? j2k_dev::SMALL_T : j2k_dev::DWT_T), kMaxCtas));
+    cfg.blockDim = dim3(j2k_dev::DWT_THREADS);
+    cfg.stream = st;
+    cfg.attrs = &early;
+    cfg.numAttrs = !first;  // the first level starts after the caller's work
+    first = false;
+    const cudaError_t e = small ? cudaLaunchKernelEx(&cfg, j2k_dev::dwt_one_level_kernel<REV, j2k_dev::SMALL_T>, P)
+                                : cudaLaunchKernelEx(&cfg, j2k_dev::dwt_one_level_kernel<REV, j2k_dev::DWT_T>, P);
+    if (e != cudaSuccess) {  // nothing was pending on entry: this error is ours
+      cudaGetLastError();
+      return J2K_ERR_CUDA;
+    }
   }
   return J2K_OK;
 }

@@ -25,10 +25,6 @@ static inline void __syncthreads() {}
 static const char *g_tile;
 static inline size_t __cvta_generic_to_shared(const void *p) { return (const char *)p - g_tile; }
 static void host_stage_copy(uint32_t to, const void *from);
-namespace cooperative_groups {
-struct Grid { void sync() {} };
-static inline Grid this_grid() { return {}; }
-}  // namespace cooperative_groups
 
 #include "../jpeg2000-decoder_b200/csrc/dwt_kernel.cuh"
 
