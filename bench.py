@@ -539,7 +539,8 @@ def run_gpu(args, rank, world, dist):
     cfg.update({"parallelism": "replicas x%d" % world, "l2": "flushed between steps (256 MB write)",
                 "bad_blocks": bad, "cuda_graph": not args.no_graph,
                 "autotuned_t1": ({"form": T1_FORMS.get(tuned["t1_form"], "auto"),
-                                  "warps_per_cta": tuned["t1_warps_per_cta"]} if tuned else None),
+                                  "warps_per_cta": tuned["t1_warps_per_cta"] if tuned["t1_form"] == 1 else 1}
+                                 if tuned else None),
                 "autotuned_dwt": ({"coarse_levels": "one shared-memory kernel" if tuned["dwt_coarse"] == 1
                                    else "one launch per level",
                                    "candidates": ["coarse levels (<= 64 a side) in one kernel",

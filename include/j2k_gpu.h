@@ -146,7 +146,9 @@ int j2k_gpu_last_launches(const j2k_gpu_ctx *ctx, int *launches);
 
 /* Tuning knobs picked by the autotuner (0 = default). */
 typedef struct j2k_gpu_tuning {
-  int t1_warps_per_cta;  /* code-blocks decoded concurrently per CTA */
+  int t1_warps_per_cta;  /* most code-blocks decoded concurrently per CTA of the compact form, up to
+                            8; a queue too short to fill that is spread over all SMs, and the
+                            latency form has one a CTA, whatever this says */
   int dwt_tile;          /* output tile edge of the DWT level kernels (64; other values are refused) */
   int use_graph;         /* capture Tier-1 + DWT launches of a batch into a CUDA graph */
   int t1_form;           /* Tier-1 kernel form: 0 auto, 1 compact (one block per warp, throughput),
@@ -164,14 +166,15 @@ typedef struct j2k_gpu_tuning {
 int j2k_gpu_set_tuning(j2k_gpu_ctx *ctx, const j2k_gpu_tuning *t);
 int j2k_gpu_get_tuning(const j2k_gpu_ctx *ctx, j2k_gpu_tuning *t);
 /* Autotuner: times the staged batch (`iters` runs after one warm-up run per candidate)
- * under the compact and latency Tier-1 kernel forms and CTA widths (2, 4, 8 warps) and
- * records the fastest for batches of this many code-blocks (power-of-two bucket); the
- * auto form (t1_form 0) then uses it for every later batch in that bucket.  Then, with that
- * Tier-1 shape, it times the inverse DWT with the coarse levels fused into one
- * shared-memory kernel and with one launch per level (re-staging the batch for each) and
- * keeps the faster for dwt_coarse 0.  The context's own tuning is left as it was and the
- * batch is staged again with it; `best` / `best_ms` (may be NULL) receive the winner and
- * its Tier-1 time.  The staged batch can be run again afterwards. */
+ * under the compact Tier-1 kernel form with CTA widths of 2, 4 and 8 warps (those that make
+ * a difference to this batch) and under the latency form, and records the fastest for
+ * batches of this many code-blocks (power-of-two bucket); the auto form (t1_form 0) then
+ * uses it for every later batch in that bucket.  The width beside the latency form means
+ * nothing.  Then, with that Tier-1 shape, it times the inverse DWT with the coarse levels
+ * fused into one shared-memory kernel and with one launch per level (re-staging the batch
+ * for each) and keeps the faster for dwt_coarse 0.  The context's own tuning is left as it
+ * was and the batch is staged again with it; `best` / `best_ms` (may be NULL) receive the
+ * winner and its Tier-1 time.  The staged batch can be run again afterwards. */
 int j2k_gpu_autotune(j2k_gpu_ctx *ctx, void *stream, int iters, j2k_gpu_tuning *best, float *best_ms);
 
 /* Inverse DWT of one tile-component that allocates no device memory, for callers that

@@ -34,6 +34,7 @@
 #include "host_copy.h"
 #include "t1_kernel.cuh"
 #include "t1_lanes.cuh"
+#include "t1_shape.h"
 
 using namespace j2k_dev;
 
@@ -461,10 +462,7 @@ void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, c
                   const uint32_t *seg, int warps_per_cta) {
   typedef T1Layout<MAXW, MAXH> Lay;
   int best_w = 1, best_ctas = 1, best_warps = 0;
-  // a queue shorter than the resident warps is spread over all SMs: its time is that of its
-  // longest blocks, which two warps of one scheduler would lengthen (the latency form always is)
-  const int spread = std::max(1, (n + c->sm_count - 1) / c->sm_count);
-  const int wmax = LATENCY ? 1 : std::min(spread, warps_per_cta > 0 ? std::min(8, warps_per_cta) : 8);
+  const int wmax = j2k::t1_most_warps(LATENCY ? j2k::T1_LATENCY : j2k::T1_COMPACT, warps_per_cta, n, c->sm_count);
   for (int w = 1; w <= wmax; ++w) {
     const size_t sm = sizeof(T1Tables) + (size_t)w * Lay::PER_WARP;
     if (sm > c->smem_optin) break;
@@ -489,14 +487,7 @@ void launch_t1_as(j2k_gpu_ctx *c, cudaStream_t st, int n, const j2k_cblk *cbs, c
 // Tier-1 form for a batch of n code-blocks: 1 compact warp form (throughput), 2 latency
 // warp form, 3 one block per lane, and warps per CTA of a warp form.  An explicit
 // tuning.t1_form wins; the auto form (0) takes the autotuned choice of the queue's size
-// bucket, else the latency form while the queue holds at most `t1_latency_waves` blocks
-// per resident warp slot of the GPU, and for longer queues while the serial chain of the
-// longest block still dominates: the compact form takes twice as long for it, and that is
-// paid back only once the whole queue takes about 2.2 times as long as the chain.  Measured Tier-1
-// ms, latency / compact form: 4096x2160 12-bit 9/7 pictures x2 3.95 / 7.27, x4 6.25 / 8.22, x6
-// 9.27 / 9.98; 2048x2048 9/7 x8 4.43 / 8.05; 1080p 9/7 frames x8 3.90 / 4.01, x10 4.82 / 4.50,
-// x24 11.46 / 9.58; 1080p lossless x6 12.54 / 12.29.  (Chain: 0.73 us a coded byte and 34 us a
-// pass; the compact form takes 1.3 MB of coded bytes a ms.)  The lane form is only taken
+// bucket, else the rule of t1_auto_form (t1_shape.h).  The lane form is only taken
 // when asked for: on B200 it measured 4.2x slower than the compact form on 1080p 9/7
 // frames (its lanes' pass walks diverge: 4.4 of 32 threads active per instruction).
 void t1_shape(const j2k_gpu_ctx *c, int n, int &form, int &warps) {
@@ -512,8 +503,7 @@ void t1_shape(const j2k_gpu_ctx *c, int n, int &form, int &warps) {
     return;
   }
   const int waves = c->tuning.t1_latency_waves > 0 ? c->tuning.t1_latency_waves : 2;
-  const double chain_us = 0.73 * c->sg.longest + 34.0 * c->sg.longest_passes, queue_us = c->sg.coded / 1300.0;
-  form = (long long)n <= (long long)waves * c->sm_count * 32 || queue_us < 2.2 * chain_us ? 2 : 1;
+  form = j2k::t1_auto_form(n, waves, c->sm_count, c->sg.coded, c->sg.longest, c->sg.longest_passes);
 }
 
 // Enqueue the Tier-1 stage: the lane kernel on the lane queue and a warp form on the rest,
@@ -1266,30 +1256,27 @@ extern "C" int j2k_gpu_autotune(j2k_gpu_ctx *c, void *stream, int iters, j2k_gpu
   const int bucket = n > 0 ? 31 - __builtin_clz((unsigned)n) : 0;
   j2k_gpu_ctx::TuneEntry win;
   win.t1_ms = 1e30f;
-  static const int forms[2] = {1, 2};
-  static const int widths[3] = {2, 4, 8};
-  for (int f : forms)
-    for (int w : widths) {
-      j2k_gpu_tuning t = saved;
-      t.t1_form = f;
-      t.t1_warps_per_cta = w;
-      t.use_graph = 0;
-      int rc = j2k_gpu_set_tuning(c, &t);
-      float tmin = 1e30f;
-      for (int i = 0; rc == J2K_OK && i <= iters; ++i) {
-        if ((rc = j2k_gpu_batch_run(c, stream)) != J2K_OK || (rc = j2k_gpu_batch_sync(c, -1)) != J2K_OK) break;
-        if (i > 0) tmin = std::min(tmin, c->t_t1);  // the first run warms caches and clocks
-      }
-      if (rc != J2K_OK) {
-        c->tuning = saved;
-        return rc;
-      }
-      if (tmin < win.t1_ms) {
-        win.t1_ms = tmin;
-        win.form = f;
-        win.warps = w;
-      }
+  for (const j2k::T1Shape &shape : j2k::t1_candidates(n, c->sm_count)) {
+    j2k_gpu_tuning t = saved;
+    t.t1_form = shape.form;
+    t.t1_warps_per_cta = shape.warps;
+    t.use_graph = 0;
+    int rc = j2k_gpu_set_tuning(c, &t);
+    float tmin = 1e30f;
+    for (int i = 0; rc == J2K_OK && i <= iters; ++i) {
+      if ((rc = j2k_gpu_batch_run(c, stream)) != J2K_OK || (rc = j2k_gpu_batch_sync(c, -1)) != J2K_OK) break;
+      if (i > 0) tmin = std::min(tmin, c->t_t1);  // the first run warms caches and clocks
     }
+    if (rc != J2K_OK) {
+      c->tuning = saved;
+      return rc;
+    }
+    if (tmin < win.t1_ms) {
+      win.t1_ms = tmin;
+      win.form = shape.form;
+      win.warps = shape.warps;
+    }
+  }
   c->tune_table[bucket] = win;
   // DWT: the coarse levels in one shared-memory kernel, or one launch per level.  The choice
   // shapes the staged task tables, so each candidate re-stages the batch; the winner is kept
