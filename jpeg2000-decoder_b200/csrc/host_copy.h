@@ -5,7 +5,9 @@
  * fault every 4 KB): the 53 MB of a 4096x2160 48-bit picture took 11.1 ms of a 21 ms call.
  * Eight threads on pieces of 1 MB take 2.6 ms.  Smaller pictures mostly land in memory that the
  * allocator hands out again without faults, where one thread is as fast (12.6 MB: 0.65 against
- * 0.52 ms), so the threads start at 16 MB.
+ * 0.52 ms), so the threads start at 16 MB.  All calls of the process together have at most
+ * COPY_HELPERS threads beside their callers (two large copies at full speed): a service whose
+ * clients all wait for large pictures would start seven threads for each of them.
  */
 #ifndef J2K_HOST_COPY_H
 #define J2K_HOST_COPY_H
@@ -19,7 +21,28 @@
 namespace j2k {
 
 constexpr size_t COPY_PIECE = (size_t)1 << 20, COPY_THREADED_FROM = (size_t)16 << 20;
-constexpr int COPY_THREADS = 8;
+constexpr int COPY_THREADS = 8, COPY_HELPERS = 2 * (COPY_THREADS - 1);
+
+// Helper threads that a call may start, out of those no other call holds
+class CopyHelpers {
+ public:
+  explicit CopyHelpers(int want) : n_(0) {
+    int left = free_().load();
+    do n_ = std::max(0, std::min(want, left));
+    while (n_ && !free_().compare_exchange_weak(left, left - n_));
+  }
+  ~CopyHelpers() { free_().fetch_add(n_); }
+  CopyHelpers(const CopyHelpers &) = delete;
+  CopyHelpers &operator=(const CopyHelpers &) = delete;
+  int count() const { return n_; }
+
+ private:
+  static std::atomic<int> &free_() {
+    static std::atomic<int> n{COPY_HELPERS};
+    return n;
+  }
+  int n_;
+};
 
 // Calls piece(thread, offset, length) for every piece of `bytes`; `thread` is below
 // COPY_THREADS and no two calls with the same one overlap.  Returns false when a call did, after
@@ -28,7 +51,8 @@ template <class F>
 bool copy_in_pieces(size_t bytes, F piece) {
   const size_t pieces = (bytes + COPY_PIECE - 1) / COPY_PIECE;
   const unsigned cores = std::thread::hardware_concurrency();
-  const int n = (int)std::min<size_t>({(size_t)COPY_THREADS, pieces, std::max<size_t>(1, cores)});
+  const CopyHelpers helpers((int)std::min<size_t>({(size_t)COPY_THREADS, pieces, std::max<size_t>(1, cores)}) - 1);
+  const int n = 1 + helpers.count();
   std::atomic<bool> ok{true};
   std::atomic<size_t> next{0};
   auto work = [&](int t) {
