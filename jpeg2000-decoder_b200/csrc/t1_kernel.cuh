@@ -179,9 +179,13 @@ __device__ __forceinline__ void mq_init(Mq &m, const uint8_t *base, uint32_t len
 // One symbol (MQ_DECODE, bmi_mq_decoder.h:86-128) of a context whose slot entry is `e`, T being
 // at least 0; returns the symbol in bit 31 (the other bits mean nothing: callers test the sign,
 // which takes no instruction to extract) and leaves the entry that follows in `e` and in the
-// slot.  The
-// throughput form returns early on an MPS without renormalisation; the latency form has no
-// branch: the successor (itself, after an MPS, after an LPS) is one of the state's records.
+// slot.  The throughput form returns early on an MPS without renormalisation; the latency form has
+// no branch: the successor (itself, after an MPS, after an LPS) is one of the state's records.
+// All lanes decode the same symbols from the same registers and store the same entry, so a slot's
+// load and store need the warp in lock-step between them: no branch from here to the next
+// warp-wide operation may depend on the lane.  Stores that only some lanes make are predicated
+// (put_sample, flip_sample, put_label), and the passes meet at __syncwarp() for every chunk, every
+// sample that becomes significant and every list of refinement symbols.
 template <bool LATENCY>
 __device__ __forceinline__ uint32_t mq_symbol(Mq &m, uint8_t *slot, uint2 &e, const uint8_t *tab) {
   const int32_t q = (int32_t)e.x;
@@ -680,6 +684,7 @@ __device__ __forceinline__ void refine(const Block &b, const uint8_t *list, int 
     }
   }
 singles:
+  __syncwarp();  // the ways here differ in length
   // one at a time: the throughput form, a chunk's last three, and while a carry waits
   for (; i < n; ++i) {
     bits = push(bits, mq_decode<LATENCY>(mq, cx, list[i], b.mq));
@@ -725,6 +730,7 @@ __device__ __forceinline__ void refinement_pass(const Block &b, int p, Mq &mq, R
       rf.z |= rows.z;
       rf.w |= rows.w;
       if (lane == 0) b.rf[s * chunks + h] = rf;
+      __syncwarp();
       if (RAW) {
         for (int i = 0; i < n; i += 32) b.bits[i >> 5] = raw_bits(raw, min(32, n - i));
       } else {
