@@ -93,13 +93,10 @@ __device__ __forceinline__ int mirror(int p, int n) {
   return p;
 }
 
-// Where that sample lies on the de-interleaved line, whose low part has lo samples.  The part
-// follows from the mirrored position: the only sample of a line of one is its low part, whatever
-// the parity of p.
-__device__ __forceinline__ int window_source(int p, int n, int lo) {
-  const int x = mirror(p, n);
-  return ((x & 1) ? lo : 0) + (x >> 1);
-}
+// Where the part that holds a parity's samples begins on the de-interleaved line, whose low part
+// has lo samples: sample mirror(p, n) lies at part_start(p & 1, n, lo) + (mirror(p, n) >> 1).  A
+// line of one sample has only its low part, for odd positions as well.
+__device__ __forceinline__ int part_start(int odd, int n, int lo) { return odd && n > 1 ? lo : 0; }
 
 __device__ __forceinline__ float lift97(float s, float c, float l, float r) {
   return __fsub_rn(s, __fmul_rn(c, __fadd_rn(l, r)));
@@ -219,12 +216,12 @@ __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const W
   const int odd = lane & 1, high = warp & 1;
   int col[COLS];
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) col[j] = window_source(ox - DWT_H + lane + 32 * j, rw, lw);
+  for (int j = 0; j < COLS; ++j) col[j] = (mirror(ox - DWT_H + lane + 32 * j, rw) >> 1) + part_start(odd, rw, lw);
   const bool last = lane < N - 32 * (COLS - 1);
   const bool inside = oy >= DWT_H && oy + TILE + DWT_H <= rh;
   for (int w = 0; w < nw; ++w) {
     const bool ll = !high && !odd;
-    const T *base = ll ? src[w].llsrc : src[w].quad;
+    const T *base = ll ? src[w].llsrc : src[w].quad + (size_t)part_start(high, rh, lh) * src[w].stride_q;
     const int stride = ll ? src[w].stride_ll : src[w].stride_q;
     const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(S[w].tile + warp * PITCH + lane);
     auto copy = [&](const T *line, uint32_t d) {
@@ -233,14 +230,14 @@ __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const W
         if (j < COLS - 1 || last) stage_copy(d + 128 * j, line + col[j]);
     };
     if (inside) {
-      const T *line = base + (size_t)window_source(oy - DWT_H + warp, rh, lh) * stride;
+      const T *line = base + (size_t)((oy - DWT_H + warp) >> 1) * stride;
       const size_t step = (size_t)(WARPS / 2) * stride;
 #pragma unroll
       for (int i = 0; i < N / WARPS; ++i, line += step) copy(line, d0 + 4 * PITCH * WARPS * i);
     } else {
 #pragma unroll 1
       for (int i = 0; i < N / WARPS; ++i)
-        copy(base + (size_t)window_source(oy - DWT_H + warp + WARPS * i, rh, lh) * stride, d0 + 4 * PITCH * WARPS * i);
+        copy(base + (size_t)(mirror(oy - DWT_H + warp + WARPS * i, rh) >> 1) * stride, d0 + 4 * PITCH * WARPS * i);
     }
   }
 }
