@@ -9,8 +9,8 @@
  * lifting eight outputs at a time in registers, and stores the 64x64 result from the column
  * pass.  Every level is one read and one write of the level's samples; all tile-components
  * of a batch at a given level share one launch.
- * The kernels are bound by instruction issue and the latency of a tile's phases (59 % of the
- * issue slots in the 4096x2160 level, DRAM 1.3 TB/s), so the work is cut into short independent
+ * The kernels are bound by instruction issue and the latency of a tile's phases (a 4096x2160 level:
+ * 61 % of the issue slots of an active SM, DRAM 1.4 TB/s), so the work is cut into short independent
  * chains, the staging walks lines with pointers, and a tile's copies run under the column pass
  * of the tile before it.  Measured on B200 against a thread per 72-sample line streamed through
  * shared memory: a 4096x2160 9/7 plane of five levels 75.4 -> 43.3 us, a 1000x777 5/3 tile
@@ -205,7 +205,8 @@ __device__ __forceinline__ void stage_copy(uint32_t to, const T *from) {
 // take LL, the others the level's quadrants (a line of one sample has only its low part, which
 // odd positions then read as well; no output comes from them), and inside the level a warp's
 // pointers advance by whole lines.
-template <bool REV, int TILE>
+enum { STAGE_DETAIL = 1, STAGE_LL = 2 };  // the quadrants to stage
+template <bool REV, int TILE, int WHICH = STAGE_DETAIL | STAGE_LL>
 __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const WinSrc<REV> *src, int rw, int rh, int lw,
                                           int lh, int ox, int oy) {
   typedef typename DwtTypes<REV>::T T;
@@ -214,6 +215,7 @@ __device__ __forceinline__ void dwt_stage(DwtSmem<REV, TILE> *S, int nw, const W
   static_assert(DWT_THREADS == FUSED_THREADS && WARPS % 2 == 0 && N % WARPS == 0, "rows are dealt to an even number of warps");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int odd = lane & 1, high = warp & 1;
+  if (!(WHICH & (odd || high ? STAGE_DETAIL : STAGE_LL))) return;
   int col[COLS];
 #pragma unroll
   for (int j = 0; j < COLS; ++j) col[j] = (mirror(ox - DWT_H + lane + 32 * j, rw) >> 1) + part_start(odd, rw, lw);
@@ -424,22 +426,24 @@ struct LevelArgs {
   int stride_out, rw, rh, lw, lh, ox, oy;  // (ox, oy): the tile
   bool ll_gain, refcompat;
 };
+template <bool REV, int TILE, int WHICH = STAGE_DETAIL | STAGE_LL>
+__device__ __forceinline__ void dwt_stage_tile(LevelSmem<REV, TILE> &S, const LevelArgs<REV> &a) {
+  dwt_stage<REV, TILE, WHICH>(&S.win, 1, &a.src, a.rw, a.rh, a.lw, a.lh, a.ox, a.oy);
+}
 // Output tiles of levels, stored to their `out`, one after the other: next(args) sets the next
 // tile's arguments or returns false.  The copies of a tile's window run under the column pass of
-// the tile before it.
-template <bool REV, int TILE, class Next>
-__device__ __forceinline__ void dwt_tiles(LevelSmem<REV, TILE> &S, float gain, Next next) {
+// the tile before it; the first one's are started by first(args).
+template <bool REV, int TILE, class Next, class First>
+__device__ __forceinline__ void dwt_tiles(LevelSmem<REV, TILE> &S, float gain, Next next, First first) {
   LevelArgs<REV> cur, ahead;
   bool more = next(cur);
-  if (more) dwt_stage<REV, TILE>(&S.win, 1, &cur.src, cur.rw, cur.rh, cur.lw, cur.lh, cur.ox, cur.oy);
+  if (more) first(cur);
   while (more) {
     bool then = false;
     dwt_windows<REV, true, TILE>(&S.win, 1, &cur.src, cur.rw, cur.rh, cur.lw, cur.lh, cur.ll_gain, gain, cur.refcompat,
                                  cur.ox, cur.oy, S.mid, cur.out, cur.stride_out, true, [&] {
                                    then = next(ahead);
-                                   if (then)
-                                     dwt_stage<REV, TILE>(&S.win, 1, &ahead.src, ahead.rw, ahead.rh, ahead.lw, ahead.lh,
-                                                          ahead.ox, ahead.oy);
+                                   if (then) dwt_stage_tile<REV, TILE>(S, ahead);
                                  });
     cur = ahead;
     more = then;
@@ -470,7 +474,7 @@ __global__ void __launch_bounds__(DWT_THREADS) dwt_level_kernel(const DwtLevel *
     a.ll_gain = L.ll_gain != 0;
     a.refcompat = L.refcompat != 0;
     return true;
-  });
+  }, [&](const LevelArgs<REV> &a) { dwt_stage_tile<REV, DWT_T>(S, a); });
 }
 
 // ------------------------------------------------------------------ output stage -------
@@ -841,19 +845,19 @@ struct OneLevel {
 // each CTA for a shorter time (the 1000x777 level, 208 large tiles: a 5/3 tile-component of that
 // size takes 16.6 us, 19.0 with large ones; 4096x2160 with 560 and 2176 tiles is left as it is).
 constexpr int SMALL_T = 32, SMALL_MOST = 2 * 148;
-// The next level's CTAs may be launched while this one drains (programmatic launch) and wait here
-// for its results, so a level costs no launch latency: 256x256, 1000x777 and 4096x2160 planes of
-// five levels take 24.8, 28.5 and 57.3 us from call to result, against 33.6, 36.3 and 64.5 with
-// plain launches and 27.4, 32.4 and 58.7 as one cooperative launch (calls one behind the other,
-// inputs not in L2, last two: 18.5 and 47.4 us, cooperative 18.7 and 46.9).  No CTA waits for one
-// that is not yet running, so the levels need no part of the GPU to themselves, as a cooperative
-// launch does: that is refused where the caller may use fewer SMs, and waits until work on other
-// streams has left every SM room.
+// The next level's CTAs may be launched while this one drains (programmatic launch): their first
+// detail quadrants, which no level writes, are on their way when they wait for this one's results,
+// so a level costs no launch latency.  256x256, 1000x777 and 4096x2160 tile-components of five
+// levels take 27, 30 and 58 us from call to result, against 34, 36 and 65 with plain launches and
+// 30, 34 and 61 as one cooperative launch; called one behind the other with inputs not in L2 18,
+// 18.5 and 45.5 us, cooperative 15, 18.7 and 47.2 (the smallest is then bound by the host's five
+// launches).  No CTA waits for one that is not yet running, so the levels need no part of the GPU
+// to themselves, as a cooperative launch does: that is refused where the caller may use fewer SMs,
+// and waits until work on other streams has left every SM room.
 template <bool REV, int TILE>
 __global__ void __launch_bounds__(DWT_THREADS) dwt_one_level_kernel(const OneLevel<REV> L) {
   __shared__ LevelSmem<REV, TILE> S;
   if (L.more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int tiles_x = (L.rw + TILE - 1) / TILE, tiles = tiles_x * ((L.rh + TILE - 1) / TILE);
   int t = blockIdx.x;
   dwt_tiles<REV, TILE>(S, L.ll_gain, [&](LevelArgs<REV> &a) {
@@ -862,6 +866,10 @@ __global__ void __launch_bounds__(DWT_THREADS) dwt_one_level_kernel(const OneLev
          (t / tiles_x) * TILE, L.scale_ll != 0, L.refcompat != 0};
     t += gridDim.x;
     return true;
+  }, [&](const LevelArgs<REV> &a) {
+    dwt_stage_tile<REV, TILE, STAGE_DETAIL>(S, a);
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // every CTA has a tile, so every CTA waits
+    dwt_stage_tile<REV, TILE, STAGE_LL>(S, a);
   });
 }
 

@@ -149,7 +149,7 @@ __device__ __forceinline__ void t1_body(const j2k_cblk *__restrict__ cbs, const 
 
 // The two kernel forms.  The throughput (compact) form keeps the default register target,
 // which leaves room for 32 resident warps per SM; the latency form (batches that fit about two
-// waves) may use more registers, as occupancy does not bound it (17 warps per SM at 117; at 76
+// waves) may use more registers, as occupancy does not bound it (16 warps per SM at 117; at 76
 // to 90 it takes 3 to 8 % longer), and has one warp a CTA: its shared-memory addresses are
 // constants then (one 2048x2048 RGB 9/7 picture 3.86 -> 3.63 ms, one 256x256 picture 1.14 ->
 // 1.04 ms against CTAs of eight warps).
@@ -933,7 +933,7 @@ int enqueue_decode(j2k_gpu_ctx *c, cudaStream_t st, bool capturing) {
   const DwtLevel *d_lev = (const DwtLevel *)(D + o_lev);
   const DwtTask *d_dtk = (const DwtTask *)(D + o_dtk);
   const float llg = j2k::irrev_ll_gain();
-  const int dwt_cap = c->sm_count * 32;  // grid-stride cap: about three waves of resident CTAs
+  const int dwt_cap = c->sm_count * 32;  // grid-stride cap: six (level kernels) to eleven (fused) waves of resident CTAs
   for (int k = 0; k < 2; ++k) {
     const int n = (int)G.n_ctasks[k];
     if (!n) continue;

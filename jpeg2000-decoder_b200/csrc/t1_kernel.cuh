@@ -6,11 +6,11 @@
  *
  * The arithmetic decode is a serial chain: every symbol needs the interval the previous one
  * left.  It bounds the kernel twice over: a single picture lasts as long as the chain of its
- * densest block (about 42 warp instructions a symbol at 4.4 cycles each; integer instructions
- * issue every second cycle, a dependent one after 4 to 5, a shared-memory load returns after
- * 23, a branch costs 15 to 25 and one on which the lanes differ 40 and more), and a long queue
- * fills the SMs' issue slots with instructions that all 32 lanes execute alike.  So what counts
- * is instructions and branches per symbol:
+ * densest block (139 cycles a symbol: 3.2 ms for the 45.3 k symbols of a 2048x2048 RGB 9/7
+ * picture's; integer instructions issue every second cycle, a dependent one after 4 to 5, a
+ * shared-memory load returns after 23, a branch costs 15 to 25 and one on which the lanes differ
+ * 40 and more), and a long queue fills the SMs' issue slots with instructions that all 32 lanes
+ * execute alike.  So what counts is instructions and branches per symbol:
  *   - the code register is extended by 32 and more bits of upcoming code, refilled four bytes at
  *     a time, so renormalisation is a shift without a loop, and one check covers two symbols;
  *   - each MQ context slot holds its probability-table entry (Qe, MPS, place in the table), so
@@ -428,14 +428,6 @@ __device__ __forceinline__ int list_positions(uint32_t x, int lane, int &pos, ui
   return __popc(rows.x) + __popc(rows.y) + __popc(rows.z) + __popc(rows.w);
 }
 
-// Significance propagation (bmi_block_decoder.cpp:10-215): samples not yet significant with a
-// significant neighbour.  Cleanup (:351-586): every sample not yet coded in this bit-plane; an
-// all-zero column is one run-length symbol (if it is 1, two uniform symbols give the row of
-// the first significant sample, whose sign follows directly).  A sample that becomes
-// significant changes the words around it, so the walk goes column by column from the words
-// themselves; the lanes only tell which columns of a chunk have work, and a column right of a
-// new significant sample joins them.
-// PASS and RAW (a bypass segment: raw bits instead of MQ symbols) are compile-time constants.
 // Predicated stores without a branch (a branch on which the lanes differ costs the warp tens
 // of cycles): a sample's first value, from the lane that owns its column (the same lane issues
 // the sample's refinements, so its updates stay in order), a refinement, and a list label
@@ -473,6 +465,14 @@ __device__ __forceinline__ uint32_t pass_rows(uint32_t word) {
   return ~((word >> SIG_POS) | (word >> CHI_POS) | (word >> PI_POS)) & ROWS;
 }
 
+// Significance propagation (bmi_block_decoder.cpp:10-215): samples not yet significant with a
+// significant neighbour.  Cleanup (:351-586): every sample not yet coded in this bit-plane; an
+// all-zero column is one run-length symbol (if it is 1, two uniform symbols give the row of
+// the first significant sample, whose sign follows directly).  A sample that becomes
+// significant changes the words around it, so the walk goes column by column from the words
+// themselves; the lanes only tell which columns of a chunk have work, and a column right of a
+// new significant sample joins them.
+// PASS and RAW (a bypass segment: raw bits instead of MQ symbols) are compile-time constants.
 template <bool LATENCY, int PASS, bool RAW>
 __device__ __forceinline__ void significance_pass(const Block &b, int p, Mq &mq, Raw &raw) {
   const int lane = b.lane;
