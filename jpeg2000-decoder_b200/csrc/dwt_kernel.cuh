@@ -10,11 +10,11 @@
  * pass.  Every level is one read and one write of the level's samples; all tile-components
  * of a batch at a given level share one launch.
  * The kernels are bound by instruction issue and the latency of a tile's phases (a 4096x2160 level:
- * 61 % of the issue slots of an active SM, DRAM 1.4 TB/s), so the work is cut into short independent
+ * 67 % of the issue slots of an active SM, DRAM 1.3 TB/s), so the work is cut into short independent
  * chains, the staging walks lines with pointers, and a tile's copies run under the column pass
  * of the tile before it.  Measured on B200 against a thread per 72-sample line streamed through
- * shared memory: a 4096x2160 9/7 plane of five levels 75.4 -> 43.3 us, a 1000x777 5/3 tile
- * 43.8 -> 16.6 us (a programmatic launch per level, 32x32 tiles in the small levels), the DWT +
+ * shared memory: a 4096x2160 9/7 plane of five levels 79.8 -> 45.4 us, a 1000x777 5/3 tile
+ * 45.1 -> 18.4 us (a programmatic launch per level, 32x32 tiles in the small levels), the DWT +
  * MCT stage of 32 1080p frames 0.955 -> 0.79 ms.
  *
  * Arithmetic follows the reference exactly so that results are bit-identical:
@@ -843,7 +843,8 @@ struct OneLevel {
 };
 // A level of at most two 64x64 tiles an SM is cut into 32x32 tiles: more of the chip works on it,
 // each CTA for a shorter time (the 1000x777 level, 208 large tiles: a 5/3 tile-component of that
-// size takes 16.6 us, 19.0 with large ones; 4096x2160 with 560 and 2176 tiles is left as it is).
+// size, in L2, takes 16.6 us, 19.0 with large ones; 4096x2160 with 560 and 2176 tiles is left as
+// it is).
 constexpr int SMALL_T = 32, SMALL_MOST = 2 * 148;
 // The next level's CTAs may be launched while this one drains (programmatic launch): their first
 // detail quadrants, which no level writes, are on their way when they wait for this one's results,
