@@ -13,8 +13,8 @@
  * 67 % of the issue slots of an active SM, DRAM 1.3 TB/s), so the work is cut into short independent
  * chains, the staging walks lines with pointers, and a tile's copies run under the column pass
  * of the tile before it.  Measured on B200 against a thread per 72-sample line streamed through
- * shared memory: a 4096x2160 9/7 plane of five levels 79.8 -> 45.4 us, a 1000x777 5/3 tile
- * 45.1 -> 18.4 us (a programmatic launch per level, 32x32 tiles in the small levels), the DWT +
+ * shared memory: a 4096x2160 9/7 plane of five levels 79.8 -> 43.2 us, a 1000x777 5/3 tile
+ * 45.1 -> 16.9 us (a programmatic launch per level, 32x32 tiles in the small levels), the DWT +
  * MCT stage of 32 1080p frames 0.955 -> 0.79 ms.
  *
  * Arithmetic follows the reference exactly so that results are bit-identical:
@@ -838,7 +838,8 @@ struct OneLevel {
   const T *coef, *ll;  // Mallat layout (row stride coef_stride) and the LL quadrant (ll_stride)
   T *out;
   int coef_stride, ll_stride, out_stride, rw, rh, lw, lh;
-  int scale_ll, refcompat, more;  // more: another level follows
+  int scale_ll, refcompat;
+  int first, more;  // the call's first launch; another level follows
   float ll_gain;
 };
 // A level of at most two 64x64 tiles an SM is cut into 32x32 tiles: more of the chip works on it,
@@ -848,16 +849,20 @@ struct OneLevel {
 constexpr int SMALL_T = 32, SMALL_MOST = 2 * 148;
 // The next level's CTAs may be launched while this one drains (programmatic launch): their first
 // detail quadrants, which no level writes, are on their way when they wait for this one's results,
-// so a level costs no launch latency.  256x256, 1000x777 and 4096x2160 tile-components of five
-// levels take 27, 30 and 58 us from call to result, against 34, 36 and 65 with plain launches and
-// 30, 34 and 61 as one cooperative launch; called one behind the other with inputs not in L2 18,
-// 18.5 and 45.5 us, cooperative 15, 18.7 and 47.2 (the smallest is then bound by the host's five
-// launches).  No CTA waits for one that is not yet running, so the levels need no part of the GPU
-// to themselves, as a cooperative launch does: that is refused where the caller may use fewer SMs,
-// and waits until work on other streams has left every SM room.
+// so a level costs no launch latency.  The first level is launched in the same way behind the
+// caller's work, and waits for it before it reads anything.  84x1088, 256x256, 1000x777 and
+// 4096x2160 tile-components of three to five levels, calls one behind the other with inputs not in
+// L2: 8.3, 12.5, 17.1 and 43.5 us (as one cooperative launch 10.4, 14.5, 18.6 and 46.6; first level
+// launched plainly 10.4, 14.4, 18.6 and 45.5); from call to result 22, 26, 31 and 58 us (cooperative
+// 22.5, 27, 30.5 and 59; the last three with plain launches 34, 36 and 65).  No CTA waits for one
+// that is not yet running, so the levels need no part of the GPU to themselves, as a cooperative
+// launch does: that is refused where the caller may use fewer SMs, and waits until work on other
+// streams has left every SM room.
 template <bool REV, int TILE>
 __global__ void __launch_bounds__(DWT_THREADS) dwt_one_level_kernel(const OneLevel<REV> L) {
   __shared__ LevelSmem<REV, TILE> S;
+  // the caller's work before the call, before anything is read and before a second level may start
+  if (L.first) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (L.more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tiles_x = (L.rw + TILE - 1) / TILE, tiles = tiles_x * ((L.rh + TILE - 1) / TILE);
   int t = blockIdx.x;

@@ -7,8 +7,9 @@
  * own arena and forbid it any other device allocation.  Those callers pass the Tier-1
  * coefficients of one tile-component and an output buffer; the intermediate resolution
  * levels live in a file-scope static device array instead of pooled buffers.  Each level is a
- * launch that overlaps the end of the one before (programmatic launch); a stream capture records
- * them like any other launches, and they run on whatever part of the GPU is free.
+ * launch that overlaps the end of the one before (programmatic launch, the first one that of the
+ * caller's work); a stream capture records them like any other launches, and they run on whatever
+ * part of the GPU is free.
  *
  * The array is J2K_NOALLOC_SCRATCH_BYTES (32 MiB) and every GPU that loads the library
  * holds it until the process exits.  In host code the array's name is only a host-side
@@ -85,7 +86,13 @@ int run_levels(const j2k_tilecomp &tc, int flags, const void *coef, void *out, i
   P.coef_stride = tc.w;
   P.refcompat = (flags & J2K_FLAG_REF_COMPAT) ? 1 : 0;
   P.ll_gain = j2k::irrev_ll_gain();
-  bool first = true;
+  // a captured first level keeps plain edges to whatever precedes it in the caller's graph
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return J2K_ERR_CUDA;
+  }
+  P.first = 1;
   for (int r = 1; r <= L; ++r) {
     P.rw = tc.res_w[r];
     P.rh = tc.res_h[r];
@@ -108,14 +115,14 @@ int run_levels(const j2k_tilecomp &tc, int flags, const void *coef, void *out, i
     cfg.blockDim = dim3(j2k_dev::DWT_THREADS);
     cfg.stream = st;
     cfg.attrs = &early;
-    cfg.numAttrs = !first;  // the first level starts after the caller's work
-    first = false;
+    cfg.numAttrs = !P.first || cap == cudaStreamCaptureStatusNone;
     const cudaError_t e = small ? cudaLaunchKernelEx(&cfg, j2k_dev::dwt_one_level_kernel<REV, j2k_dev::SMALL_T>, P)
                                 : cudaLaunchKernelEx(&cfg, j2k_dev::dwt_one_level_kernel<REV, j2k_dev::DWT_T>, P);
     if (e != cudaSuccess) {  // nothing was pending on entry: this error is ours
       cudaGetLastError();
       return J2K_ERR_CUDA;
     }
+    P.first = 0;
   }
   return J2K_OK;
 }

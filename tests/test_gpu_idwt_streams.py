@@ -1,6 +1,7 @@
 """The allocation-free inverse DWT where its callers run it: captured into a graph that is replayed
-on new coefficients, and on a stream that may use only some of the SMs.  The values are those of
-a call on an ordinary stream, bit for bit."""
+on new coefficients, on a stream that may use only some of the SMs, and behind work of the same and
+of other streams that is still running when the call is made.  The values are those of a call on an
+idle stream, bit for bit."""
 import ctypes
 
 import numpy as np
@@ -89,3 +90,43 @@ def test_stream_of_a_few_sms(pkg, rev):
     finally:
         drv.cuStreamDestroy(stream)
         drv.cuGreenCtxDestroy(green)
+
+
+@pytest.mark.parametrize("behind", ["same stream", "event", "legacy stream"])
+@pytest.mark.parametrize("rev", [0, 1])
+@pytest.mark.parametrize("w,h,levels", SHAPES)
+def test_coefficients_that_are_still_being_written(pkg, rev, w, h, levels, behind):
+    """The call sees what earlier work writes to its coefficients, and what follows it sees its
+    result: work enqueued on the same stream, work of another stream joined by an event, and work
+    of a blocking stream, which the legacy default stream waits for."""
+    import torch
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    tc = _tile(w, h, levels)
+    new, old = _coefficients(5, tc, rev), _coefficients(6, tc, rev)
+    want = torch.empty_like(new)
+    assert _call(tc, rev, new, want, 0) == 0
+    torch.cuda.synchronize()
+    src, out, after = old.clone(), torch.zeros_like(new), torch.zeros_like(new)
+    torch.cuda.synchronize()
+    err, other = rt.cudaStreamCreate()  # a blocking stream
+    assert err == rt.cudaError_t.cudaSuccess
+    writer = torch.cuda.ExternalStream(int(other))
+    caller = torch.cuda.default_stream() if behind == "legacy stream" else torch.cuda.Stream()
+    if behind == "same stream":
+        writer = caller
+    with torch.cuda.stream(caller):
+        after.fill_(1)  # a kernel right before the call
+    with torch.cuda.stream(writer):
+        torch.cuda._sleep(4000000)  # about 2 ms
+        src.copy_(new)
+        if behind == "event":
+            done = torch.cuda.Event()
+            done.record(writer)
+    if behind == "event":
+        caller.wait_event(done)
+    assert _call(tc, rev, src, out, caller.cuda_stream) == 0
+    with torch.cuda.stream(caller):
+        after.copy_(out)
+    torch.cuda.synchronize()
+    assert np.array_equal(after.cpu().numpy().view(np.int32), want.cpu().numpy().view(np.int32))
+    rt.cudaStreamDestroy(other)
